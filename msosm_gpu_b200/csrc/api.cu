@@ -93,6 +93,9 @@ cudaError_t dalloc(T **p, size_t count, size_t &total)
 // The tensor-core kernel's limit on each wait for one of its GEMMs (which
 // take microseconds): 1 s of global timer.
 constexpr long long kTcWaitLimitDefaultNs = 1000000000ll;
+// Most spans in a work item's shared-memory window (16 bytes each); shorter
+// periods refill it within a block.
+constexpr unsigned long kMaxSpanWindow = 512;
 
 }  // namespace
 
@@ -106,7 +109,6 @@ struct msosm_dedisp {
     unsigned long M = 0, N = 0, M_min = 0;
     unsigned int flags = 0;
     bool series = true;
-    bool pingpong = false;  // tuning: MSOSM_DEDISP_PINGPONG=1 selects the two-buffer kernel
     std::vector<unsigned long> Nd;
     std::vector<int> dc;
     std::vector<int> delays;  // D x N (host copy)
@@ -120,6 +122,7 @@ struct msosm_dedisp {
     float2 *ring = nullptr, *H = nullptr, *hist = nullptr, *series_buf = nullptr;
     uint16_t *delays_d = nullptr;
     float2 *tw_fwd = nullptr, *tw_inv = nullptr, *tw_inv_m = nullptr;
+    int *work = nullptr;  // the dedispersion kernel's item counter (DedispArgs::work)
     void *staging[2] = {nullptr, nullptr};
     uint32_t *u16_out = nullptr;
     // folding
@@ -174,7 +177,7 @@ void release(msosm_dedisp *d)
     void *bufs[] = {d->ring, d->H, d->hist, d->series_buf, d->delays_d, d->tw_fwd, d->tw_inv, d->tw_inv_m,
                     d->staging[0], d->staging[1], d->u16_out, d->part_main, d->part_pend, d->prof_out,
                     d->acc_main, d->acc_pend, d->span_a_d, d->span_b_d, d->span_p_d, d->span_dest_d,
-                    d->lA, d->lB, d->lI, d->tw1f, d->tw1i, d->tw2f, d->tw2i, d->status_d,
+                    d->work, d->lA, d->lB, d->lI, d->tw1f, d->tw1i, d->tw2f, d->tw2i, d->status_d,
                     d->row_max, d->h_max, d->delay_max_d};
     for (void *p : bufs)
         if (p)
@@ -235,23 +238,36 @@ msosm_status design_filters(int log2n, const std::vector<ChirpParams> &cp, float
     return MSOSM_OK;
 }
 
+int blocks_per_step(const msosm_dedisp *d)
+{
+    return d->tc ? tc_blocks_per_step(d->log2n) : dedisp_blocks_per_step(d->log2n);
+}
+
 // Whether the fused kernel keeps a work item's two profiles in shared memory
-// (else in the global partial rows): up to kMaxSmemBins bins, and in the
-// tensor-core kernels only when they fit beside the tables, operand buffers
-// and span window in the device's per-block limit (at 8192 points that is
-// 1024 bins with the usual 64-span window; at 16384, 2048).
+// (else in the global partial rows): up to kMaxSmemBins bins, when they fit
+// beside the kernel's buffers -- for the tensor-core kernels in the device's
+// per-block limit (at 8192 points that is 1024 bins with the usual 64-span
+// window; at 16384, 2048), for the FP32 kernel without costing it one of the
+// CTAs it is built for per SM (3300 bins up to 4096 points).
 bool prof_in_smem(const msosm_dedisp *d)
 {
     if (d->nbins > kMaxSmemBins)
         return false;
-    if (!d->tc)
+    if (d->large)
         return true;
-    const size_t need = tc_smem_base(d->log2n) + fold_smem_bytes(d->nbins, d->win_cap, true, tc_threads(d->log2n));
-    return need <= tc_smem_limit();
+    const size_t fs = fold_smem_bytes(d->nbins, d->win_cap, true);
+    if (d->tc)
+        return tc_smem_base(d->log2n) + fs <= tc_smem_limit();
+    return dedisp_smem(d->log2n, true, fs) <= dedisp_smem_share(d->log2n);
 }
 
-// Persistent grid of the dedispersion kernel: work items (block range,
-// trial), about eight per resident CTA, spread evenly over the waves.
+// Block ranges per trial and the persistent grid of the dedispersion kernel.
+// A work item is one (block range, trial); the grid strides over the items.
+// The ranges are chosen so that the items fill whole waves of the resident
+// CTAs: the smallest of waves x (steps of an item + kItemSteps), where
+// kItemSteps stands for an item's own work (its filter and profile rows).
+// With eight items per CTA whatever the remainder, the last wave of 128
+// trials x 2048 blocks at FFT 4096 left 8 % of the CTAs idle.
 cudaError_t plan_grid(msosm_dedisp *d)
 {
     int dev = 0, sms = 0;
@@ -260,23 +276,32 @@ cudaError_t plan_grid(msosm_dedisp *d)
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess)
         return e;
-    const int threads = d->tc ? tc_threads(d->log2n) : (int)(d->N / 16);
-    const size_t extra = d->fold ? fold_smem_bytes(d->nbins, d->win_cap, prof_in_smem(d), threads) : 0;
-    int per_sm = d->tc ? tc_blocks_per_sm(d->log2n, d->tc_bf16, d->series, d->fold, extra)
-                       : dedisp_blocks_per_sm(d->log2n, d->pingpong, d->series, d->fold, extra);
+    const size_t extra = d->fold ? fold_smem_bytes(d->nbins, d->win_cap, prof_in_smem(d)) : 0;
+    int per_sm;
+    if (d->tc) {
+        per_sm = tc_blocks_per_sm(d->log2n, d->tc_bf16, d->series, d->fold, extra);
+    } else {
+        per_sm = dedisp_ctas_per_sm(d->log2n);
+        if (dedisp_smem(d->log2n, d->fold, extra) > dedisp_smem_share(d->log2n))
+            per_sm = 1;
+    }
     if (per_sm < 1)
         per_sm = 1;
     const long long resident = (long long)per_sm * sms;
-    long long R = (8 * resident + d->D - 1) / d->D;
-    // the tensor-core kernel works in steps of a pair of blocks (one block at 16384)
-    const int bps = d->tc ? tc_blocks_per_step(d->log2n) : 1;
+    const int bps = blocks_per_step(d);
     const long long units = (d->count + bps - 1) / bps;
-    if (R > units)
-        R = units;
-    if (R < 1)
-        R = 1;
-    d->R = (int)R;
-    const long long items = (long long)d->D * R;
+    constexpr double kItemSteps = 1.5;
+    const long long r_max = std::max(1ll, std::min(units, 12 * resident / d->D + 1));
+    double best = 0.0;
+    for (long long R = 1; R <= r_max; ++R) {
+        const long long waves = ((long long)d->D * R + resident - 1) / resident;
+        const double cost = (double)waves * ((double)((units + R - 1) / R) + kItemSteps);
+        if (R == 1 || cost < best) {
+            best = cost;
+            d->R = (int)R;
+        }
+    }
+    const long long items = (long long)d->D * d->R;
     const long long waves = (items + resident - 1) / resident;
     d->grid = (int)((items + waves - 1) / waves);
     if (std::getenv("MSOSM_DEBUG_GRID"))
@@ -661,8 +686,6 @@ msosm_status msosm_dedisp_create(const float *bw, const float *dm, const float *
         }
         d->S = (int)S;
     }
-    if (const char *pp = std::getenv("MSOSM_DEDISP_PINGPONG"))
-        d->pingpong = std::atoi(pp) != 0;
 
 #define CKD(call)                                                                                      \
     do {                                                                                               \
@@ -723,6 +746,8 @@ msosm_status msosm_dedisp_create(const float *bw, const float *dm, const float *
             release(d);
             return s;
         }
+        CKD(dalloc(&d->work, 2, tot));
+        CKD(cudaMemsetAsync(d->work, 0, 2 * sizeof(int), d->stream));
         if ((s = design_filters(log2n, cp, scale, sign, d->tw_inv_m, d->tw_fwd, d->H, d->stream)) != MSOSM_OK) {
             release(d);
             return s;
@@ -910,7 +935,7 @@ static msosm_status fold_prepare(msosm_dedisp *d, int sb, FoldArgs &fa)
     fa.smem_prof = prof_in_smem(d) ? 1 : 0;
     fa.span_cap = d->win_cap;
     fa.inv_bpt = 1.0f / (float)d->bpt;
-    fa.g_shift = fold_g_shift(d->bpt, d->large ? 256 : (int)(d->N / 16));
+    fa.g_shift = fold_g_shift(d->bpt);
     return MSOSM_OK;
 }
 
@@ -1073,6 +1098,7 @@ static msosm_status call_begin(msosm_dedisp *d, const void *input, InputKind kin
     da.tw = d->tw_inv;
     da.series = d->series_buf;
     da.fold.nspans = -1;
+    da.work = d->work;
     da.status = d->status_d;
     da.wait_limit_ns = d->tc_wait_limit_ns;
     da.row_max = d->row_max;
@@ -1130,7 +1156,7 @@ static msosm_status filter_block(msosm_dedisp *d, const void *input, InputKind k
     if (d->tc)
         CK(launch_tc_dedisp(d->log2n, d->tc_bf16, d->series, d->fold, da, d->grid, d->stream));
     else
-        CK(launch_dedisp(d->log2n, d->pingpong, d->series, d->fold, da, d->grid, d->stream));
+        CK(launch_dedisp(d->log2n, d->series, d->fold, da, d->grid, d->stream));
     d->launches += 1;
     if (ev)
         CK(cudaEventRecord(ev->e[3], d->stream));
@@ -1244,8 +1270,7 @@ msosm_status msosm_batch_create(msosm_dedisp *const *handles, int n, msosm_batch
         for (int i : g.members) {
             const msosm_dedisp *d = b->h[i];
             if (g.fold)
-                g.fold_smem = std::max(g.fold_smem, fold_smem_bytes(d->nbins, d->win_cap, prof_in_smem(d),
-                                                                    tc_threads(d->log2n)));
+                g.fold_smem = std::max(g.fold_smem, fold_smem_bytes(d->nbins, d->win_cap, prof_in_smem(d)));
         }
         int per_sm = tc_blocks_per_sm(g.log2n, g.bf16, g.series, g.fold, g.fold_smem);
         if (per_sm < 1)
@@ -1450,10 +1475,9 @@ msosm_status msosm_dedisp_fold_init(msosm_dedisp *d, float period, float fs, uns
     d->out_scale = nb == ps ? 1.0 : 1.0 / (double)d->bpt;
     d->detect = detect;
     d->span_cap = (int)((unsigned long)d->count * d->M / ps) + 8;
-    // spans one block can touch: ceil(M/ps) + 2 periods
-    d->win_cap = (int)(d->M / ps) + 4;
-    if (d->win_cap < 64)
-        d->win_cap = 64;
+    // window of spans a work item holds at a time: those one block can touch
+    // (ceil(M/ps) + 2 periods), within 64 .. kMaxSpanWindow
+    d->win_cap = (int)std::min<unsigned long>(std::max<unsigned long>(d->M / ps + 4, 64), kMaxSpanWindow);
     d->fold = true;
     if (!d->large) {
         cudaError_t e = plan_grid(d);
@@ -1857,7 +1881,7 @@ msosm_status msosm_fold_data(msosm_fold *f)
     a.smem_prof = f->nbins <= kMaxSmemBins ? 1 : 0;
     a.span_cap = f->win_cap;
     a.inv_bpt = 1.0f / (float)f->bpt;
-    a.g_shift = fold_g_shift(f->bpt, 256);
+    a.g_shift = fold_g_shift(f->bpt);
     CK(launch_fold_series(f->I, (long long)f->size, f->R, a, f->grid, 1, f->stream));
     CK(launch_fold_reduce(f->part_main, f->part_pend, 1, f->R, f->nbins, f->acc_main, f->acc_pend, f->stream));
     // the pinned span staging is reused by the next call

@@ -1,19 +1,11 @@
-// kernels.cu -- sm_100a kernels of the MS-OSM / OSM dedispersion path.
+// kernels.cu -- sm_100a kernels of the MS-OSM / OSM dedispersion path (the
+// fused dedispersion kernels are in pair_dedisp.cu and tc_dedisp.cu).
 //
 //   forward_kernel  decode (uint16 offset-binary or complex64) + forward FFT of
 //                   the overlapping windows of one call, written into the
 //                   spectrum ring shared by all DM trials.  Replaces
 //                   uint16ToComplex + the forward cufftExecC2C
 //                   (gpu/gpu_kernel.cu:276-299, msosm_gpu_dm_concurrent.cpp:123-129).
-//   dedisp_kernel   persistent; per (DM trial, block): gather each bin's
-//                   delayed spectrum from the ring, multiply by H, inverse FFT
-//                   in shared memory, keep the second half (overlap-save
-//                   discard), then write the series and/or detect and fold.
-//                   Replaces ComplexMultiplyDelay_concurrent_batch + inverse
-//                   cufftExecC2C + DiscardSamples_concurrent_batch
-//                   (gpu/gpu_kernel.cu:128-198,236-258) and, fused, the
-//                   calculateIntensity kernel + host fold of Fold_GPU
-//                   (gpu/gpu_kernel.cu:347-353, folding/fold_gpu.cpp:48-194).
 //   design_kernel   dedispersion filter H per trial on the device: FP64 chirp
 //                   phase reduced mod 2 pi, M-point inverse FFT, zero pad,
 //                   2M-point FFT (msosm_prepare.cpp:37-84 on the host in the
@@ -109,111 +101,6 @@ __global__ void __launch_bounds__(FftShape<LOG2N>::T) forward_kernel(FwdArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// fused dedispersion + detection + folding
-// ---------------------------------------------------------------------------
-
-template <int LOG2N, bool PP, bool SERIES, bool FOLD>
-__global__ void __launch_bounds__(FftShape<LOG2N>::T) dedisp_kernel(DedispArgs a)
-{
-    using F = FftShape<LOG2N>;
-    constexpr int N = F::N, M = N / 2, T = F::T;
-    constexpr int RL = F::radix(F::NST - 1);
-    extern __shared__ float2 smem[];
-    float2 *buf0 = smem;
-    float2 *buf1 = PP ? smem + F::SMEM : smem;
-    float *ibuf = reinterpret_cast<float *>(smem + (PP ? 2 : 1) * F::SMEM);
-    FoldSmem fw;
-    if constexpr (FOLD) {
-        // after ibuf: [span window a, b, phase0, dest] [partials] [prof_main, prof_pend]
-        fold_smem_layout(fw, ibuf + ibuf_floats(M), a.fold);
-    }
-    const int tid = threadIdx.x;
-    const int items = a.D * a.R;
-    for (int w = blockIdx.x; w < items; w += gridDim.x) {
-        const int dm = w % a.D;
-        const int rr = w / a.D;
-        const int kb = (int)((long long)a.count * rr / a.R);
-        const int ke = (int)((long long)a.count * (rr + 1) / a.R);
-        const float2 *__restrict__ Hd = a.H + (size_t)dm * N;
-        const uint16_t *__restrict__ dl = a.delays + (size_t)dm * N;
-        int sp = 0, sbase = 0, scnt = 0;
-        if constexpr (FOLD) {
-            if (a.fold.smem_prof) {
-                for (int i = tid; i < 2 * a.fold.nbins; i += blockDim.x)
-                    fw.prof_main[i] = 0.f;
-            } else {
-                fw.prof_main = a.fold.part_main + (size_t)w * a.fold.nbins;
-                fw.prof_pend = a.fold.part_pend + (size_t)w * a.fold.nbins;
-            }
-            sp = span_lower_bound(a.fold.span_b, a.fold.nspans, (long long)kb * M);
-            span_refill(a.fold, fw, sp, sbase, scnt);
-        }
-        long long kg = a.k0 + kb;
-        const int smask = a.S - 1;  // the ring depth is a power of two
-        for (int k = kb; k < ke; ++k, ++kg) {
-            float2 v[16];
-            const int slot_k = (int)(kg & smask);
-            if (kg >= a.max_delay) {
-#pragma unroll
-                for (int r = 0; r < 16; ++r) {
-                    const int b = tid + r * T;
-                    const int s = (slot_k - (int)__ldg(&dl[b])) & smask;
-                    v[r] = cmul(a.ring[(size_t)s * N + b], __ldg(&Hd[b]));
-                }
-            } else {
-#pragma unroll
-                for (int r = 0; r < 16; ++r) {
-                    const int b = tid + r * T;
-                    const int d = (int)__ldg(&dl[b]);
-                    float2 x = make_float2(0.f, 0.f);
-                    if (kg >= d)  // blocks before the stream start are zero
-                        x = a.ring[(size_t)((slot_k - d) & smask) * N + b];
-                    v[r] = cmul(x, __ldg(&Hd[b]));
-                }
-            }
-            dft16<+1>(v);
-            // the previous block's last-stage loads (and fold reads of ibuf)
-            // must be done before buf0 is overwritten; with folding the
-            // barrier ahead of the fold already separates them
-            if constexpr (!FOLD)
-                __syncthreads();
-            stage_store<LOG2N, 0>(v, buf0, tid);
-            run_stages<LOG2N, +1, PP>(v, buf0, buf1, tid, a.tw);
-            // keep outputs n >= M (the last-stage slots with r >= R/2)
-#pragma unroll
-            for (int slot = 0; slot < 16; ++slot) {
-                if ((slot % RL) >= RL / 2) {
-                    const int t = last_out_index<LOG2N>(tid, slot) - M;
-                    const float2 y = v[slot];
-                    if constexpr (SERIES)
-                        a.series[(size_t)dm * a.count * M + (size_t)k * M + t] = y;
-                    if constexpr (FOLD) {
-                        const float p = y.x * y.x + y.y * y.y;
-                        ibuf[ipad(t)] = a.fold.detect ? sqrtf(p) : p;
-                    }
-                }
-            }
-            if constexpr (FOLD) {
-                __syncthreads();
-                fold_block<kIbufPadded>(a.fold, fw, ibuf, k * M, M, sp, sbase, scnt);
-            }
-        }
-        if constexpr (FOLD) {
-            __syncthreads();
-            if (a.fold.smem_prof) {
-                float *gm = a.fold.part_main + (size_t)w * a.fold.nbins;
-                float *gp = a.fold.part_pend + (size_t)w * a.fold.nbins;
-                for (int i = tid; i < a.fold.nbins; i += blockDim.x) {
-                    gm[i] = fw.prof_main[i];
-                    gp[i] = fw.prof_pend[i];
-                }
-            }
-            __syncthreads();
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
 // folding of a materialised intensity series (Fold_GPU)
 // ---------------------------------------------------------------------------
 
@@ -257,14 +144,14 @@ __global__ void __launch_bounds__(256) fold_series_kernel(const float *__restric
             fw.prof_main = f.part_main + ((size_t)w * D + d) * f.nbins;
             fw.prof_pend = f.part_pend + ((size_t)w * D + d) * f.nbins;
         }
-        int sp = span_lower_bound(f.span_b, f.nspans, kb * kFoldBlock), sbase = 0, scnt = 0;
-        span_refill(f, fw, sp, sbase, scnt);
+        FoldCursor cur;
+        cursor_init(f, fw, cur, kb * kFoldBlock);
         for (long long k = kb; k < ke; ++k) {
             const int t0 = (int)(k * kFoldBlock);
             for (int t = threadIdx.x; t < kFoldBlock; t += blockDim.x)
                 ibuf[ipad(t)] = (long long)t0 + t < n ? I[t0 + t] : 0.f;
             __syncthreads();
-            fold_block<kIbufPadded>(f, fw, ibuf, t0, kFoldBlock, sp, sbase, scnt);
+            fold_block<kIbufPadded>(f, fw, ibuf, t0, kFoldBlock, cur);
             __syncthreads();
         }
         if (f.smem_prof) {
@@ -421,13 +308,6 @@ template <int LOG2N>
 constexpr bool use_pingpong() { return LOG2N <= 12; }
 
 template <int LOG2N>
-size_t dedisp_smem_bytes(bool pp)
-{
-    using F = FftShape<LOG2N>;
-    return (pp ? 2 : 1) * F::SMEM * sizeof(float2) + ibuf_floats(F::N / 2) * sizeof(float);
-}
-
-template <int LOG2N>
 size_t fft_smem_bytes()
 {
     using F = FftShape<LOG2N>;
@@ -460,62 +340,9 @@ static cudaError_t forward_t(InputKind kind, const FwdArgs &a, cudaStream_t st)
     return cudaGetLastError();
 }
 
-size_t fold_smem_bytes(int nbins, int span_cap, bool smem_prof, int threads)
+size_t fold_smem_bytes(int nbins, int span_cap, bool smem_prof)
 {
-    return (size_t)span_cap * 4 * sizeof(int) + 2 * (size_t)threads * sizeof(float) +
-           (smem_prof ? 2 * (size_t)nbins * sizeof(float) : 0);
-}
-
-template <int LOG2N, bool PP, bool SERIES, bool FOLD>
-static auto dedisp_fn() { return dedisp_kernel<LOG2N, PP && use_pingpong<LOG2N>(), SERIES, FOLD>; }
-
-// Calls go(kernel) with the instantiation for (pp, series, fold).
-template <int LOG2N, typename G>
-static auto dedisp_select(bool pp, bool series, bool fold, G &&go)
-{
-    if (pp && use_pingpong<LOG2N>()) {
-        if (series && fold)
-            return go(dedisp_fn<LOG2N, true, true, true>());
-        if (fold)
-            return go(dedisp_fn<LOG2N, true, false, true>());
-        return go(dedisp_fn<LOG2N, true, true, false>());
-    }
-    if (series && fold)
-        return go(dedisp_fn<LOG2N, false, true, true>());
-    if (fold)
-        return go(dedisp_fn<LOG2N, false, false, true>());
-    return go(dedisp_fn<LOG2N, false, true, false>());
-}
-
-template <int LOG2N>
-static cudaError_t dedisp_t(bool pp, bool series, bool fold, const DedispArgs &a, int grid, cudaStream_t st)
-{
-    pp = pp && use_pingpong<LOG2N>();
-    const size_t sm = dedisp_smem_bytes<LOG2N>(pp) +
-                      (fold ? fold_smem_bytes(a.fold.nbins, a.fold.span_cap, a.fold.smem_prof != 0,
-                                              FftShape<LOG2N>::T) : 0);
-    return dedisp_select<LOG2N>(pp, series, fold, [&](auto k) -> cudaError_t {
-        cudaError_t e = set_smem(k, sm);
-        if (e != cudaSuccess)
-            return e;
-        k<<<grid, FftShape<LOG2N>::T, sm, st>>>(a);
-        return cudaGetLastError();
-    });
-}
-
-template <int LOG2N>
-static int dedisp_occ_t(bool pp, bool series, bool fold, size_t extra)
-{
-    pp = pp && use_pingpong<LOG2N>();
-    const size_t sm = dedisp_smem_bytes<LOG2N>(pp) + extra;
-    return dedisp_select<LOG2N>(pp, series, fold, [&](auto k) -> int {
-        int n = 0;
-        if (set_smem(k, sm) != cudaSuccess)
-            return 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, FftShape<LOG2N>::T, sm) != cudaSuccess)
-            return 0;
-        return n;
-    });
+    return (size_t)span_cap * 4 * sizeof(int) + (smem_prof ? 2 * (size_t)nbins * sizeof(float) : 0);
 }
 
 template <int LOG2N>
@@ -551,23 +378,6 @@ cudaError_t launch_forward(int log2n, InputKind kind, const FwdArgs &a, cudaStre
     MSOSM_DISPATCH(log2n, CALL)
 #undef CALL
     return cudaErrorInvalidValue;
-}
-
-cudaError_t launch_dedisp(int log2n, bool pp, bool series, bool fold, const DedispArgs &a, int grid,
-                          cudaStream_t st)
-{
-#define CALL(L) dedisp_t<L>(pp, series, fold, a, grid, st)
-    MSOSM_DISPATCH(log2n, CALL)
-#undef CALL
-    return cudaErrorInvalidValue;
-}
-
-int dedisp_blocks_per_sm(int log2n, bool pp, bool series, bool fold, size_t extra_smem)
-{
-#define CALL(L) dedisp_occ_t<L>(pp, series, fold, extra_smem)
-    MSOSM_DISPATCH(log2n, CALL)
-#undef CALL
-    return 0;
 }
 
 cudaError_t launch_design(int log2n, const DesignArgs &a, cudaStream_t st)
@@ -654,7 +464,7 @@ cudaError_t launch_fold_series(const float *I, long long n, int R, const FoldArg
                                cudaStream_t st)
 {
     const size_t sm =
-        ibuf_floats(kFoldBlock) * sizeof(float) + fold_smem_bytes(f.nbins, f.span_cap, f.smem_prof != 0, 256);
+        ibuf_floats(kFoldBlock) * sizeof(float) + fold_smem_bytes(f.nbins, f.span_cap, f.smem_prof != 0);
     cudaError_t e = set_smem(fold_series_kernel, sm);
     if (e != cudaSuccess)
         return e;

@@ -36,18 +36,20 @@ struct FoldArgs {
     int detect;   // 0 |y|^2, 1 |y|
     float *part_main, *part_pend;  // [items][nbins]
     int smem_prof;  // 1: the work item's profile rows live in shared memory
-    int span_cap;   // spans held in the shared-memory window (>= spans one block can touch)
+    int span_cap;   // spans held in the shared-memory window (refilled as the fold goes on)
     float inv_bpt;  // 1/bpt, for the exact-corrected division
     int g_shift;    // log2 of the lanes summing one bin (fold_g_shift)
 };
 
-// Lanes per bin in the fold: G ~ bpt/8, a power of two <= 32 (1 below whole warps).
-inline int fold_g_shift(int bpt, int threads)
+// log2 of the lanes that sum one bin in the fold: the smallest power of two
+// (at most a warp) that leaves a lane at most kFoldLane samples.  Fewer lanes
+// mean fewer instructions in all (each lane adds its own overhead and a
+// butterfly step), more lanes a shorter chain for the warps that have bins.
+constexpr int kFoldLane = 32;
+inline int fold_g_shift(int bpt)
 {
-    if (threads < 32)
-        return 0;
     int g = 0;
-    while (g < 5 && (8 << g) < bpt)
+    while (g < 5 && (kFoldLane << g) < bpt)
         ++g;
     return g;
 }
@@ -55,8 +57,8 @@ inline int fold_g_shift(int bpt, int threads)
 // intensity staging of one block: M samples, one pad slot per 32
 __host__ __device__ constexpr int ibuf_floats(int m) { return (m + (m >> 5) + 1) & ~1; }
 
-// Extra dynamic shared memory of the folding dedispersion kernel (threads: its block size).
-size_t fold_smem_bytes(int nbins, int span_cap, bool smem_prof, int threads);
+// Shared memory of a work item's span window and profiles.
+size_t fold_smem_bytes(int nbins, int span_cap, bool smem_prof);
 constexpr int kMaxSmemBins = 4096;
 
 struct DedispArgs {
@@ -72,6 +74,7 @@ struct DedispArgs {
     const float2 *tw;         // exp(+2 pi i e/N)
     float2 *series;           // [D][count*M] or nullptr
     FoldArgs fold;            // fold.nspans < 0: no folding
+    int *work;                // items handed out so far, CTAs done: zero before and after a launch
     // tensor-core kernel only
     int *status;              // nonzero after a timed-out wait
     long long wait_limit_ns;  // limit of each wait on a GEMM (0: give up at the first incomplete probe)
@@ -115,12 +118,15 @@ bool log2n_supported(int log2n);
 void set_error_message(const char *msg);
 
 cudaError_t launch_forward(int log2n, InputKind kind, const FwdArgs &a, cudaStream_t st);
-// pp: ping-pong shared-memory buffers (one barrier per FFT stage instead of
-// two; twice the buffer space); honoured for FFT sizes up to 4096
-cudaError_t launch_dedisp(int log2n, bool pp, bool series, bool fold, const DedispArgs &a, int grid,
-                          cudaStream_t st);
-// CTAs of the dedispersion kernel that fit on one SM (for the persistent grid)
-int dedisp_blocks_per_sm(int log2n, bool pp, bool series, bool fold, size_t extra_smem);
+// ---- FP32 dedispersion, 64 .. 16384-point transforms (pair_dedisp.cu)
+// a.R counts ranges of steps (dedisp_blocks_per_step blocks each)
+cudaError_t launch_dedisp(int log2n, bool series, bool fold, const DedispArgs &a, int grid, cudaStream_t st);
+// blocks one step transforms, CTAs the kernel is built for per SM, its dynamic
+// shared memory
+int dedisp_blocks_per_step(int log2n);
+int dedisp_ctas_per_sm(int log2n);
+size_t dedisp_smem(int log2n, bool fold, size_t fold_smem);
+size_t dedisp_smem_share(int log2n);
 cudaError_t launch_design(int log2n, const DesignArgs &a, cudaStream_t st);
 
 cudaError_t launch_fold_reduce(const float *part_main, const float *part_pend, int D, int R, int nbins,
@@ -143,8 +149,6 @@ cudaError_t launch_fold_series(const float *I, long long n, int R, const FoldArg
 
 // ---- tensor-core (tcgen05) dedispersion, 4096-, 8192- and 16384-point transforms (tc_dedisp.cu)
 bool tc_supported(int log2n);
-// threads per CTA of the tensor-core kernel (its fold group size)
-int tc_threads(int log2n);
 // blocks one step of the kernel transforms: 2 (a pair) at 4096 and 8192, 1 at 16384
 int tc_blocks_per_step(int log2n);
 // shared memory of the tensor-core kernel before its fold state (tables,

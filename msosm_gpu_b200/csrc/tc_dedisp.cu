@@ -36,6 +36,7 @@
 #include "fold_dev.cuh"
 #include "kernels.hpp"
 #include "tc_layout.hpp"
+#include "tmem.cuh"
 
 namespace msosm {
 namespace {
@@ -48,8 +49,6 @@ constexpr unsigned long long kWaitLimitNs = 1000000000ull;
 // attempt (an explicit 100 us suspend hint was 0.4-0.8 % slower)
 constexpr unsigned long long kProbeBelowNs = 100000ull;
 
-__device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -57,8 +56,6 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
 
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
 {
@@ -121,20 +118,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
     return true;
 }
 
-__device__ __forceinline__ void tmem_alloc(uint32_t dst, uint32_t ncols)
-{
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst), "r"(ncols)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish()
-{
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
-{
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-
 // D (tensor memory) = A * B (+ D when accumulate), one thread issues
 __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc,
                                         uint32_t accumulate)
@@ -176,20 +159,6 @@ __device__ __forceinline__ void tmem_ld_2x16(uint32_t ta, uint32_t tb, float (&a
         a[i] = __uint_as_float(r[i]);
         b[i] = __uint_as_float(r[16 + i]);
     }
-}
-
-// 32 words of this thread's TMEM lane, columns ta .. ta + 31 (two x16 stores), then the wait
-__device__ __forceinline__ void tmem_st_32(uint32_t ta, const uint32_t (&v)[32])
-{
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17};\n\t"
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%1], {%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32,%33};\n\t"
-        "tcgen05.wait::st.sync.aligned;" ::"r"(ta), "r"(ta + 16),
-        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
-        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]),
-        "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]),
-        "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-        : "memory");
 }
 
 // D1 re / im (x16 each) and 8 + 8 twiddle words (x8 each), one wait
@@ -643,7 +612,7 @@ __global__ void __launch_bounds__(TcShape<LOG2N>::THREADS, TcShape<LOG2N>::CTAS_
                     hreg[j] = make_float4(hreg[j].x * sc, hreg[j].y * sc, hreg[j].z * sc, hreg[j].w * sc);
             }
         }
-        int sp = 0, sbase = 0, scnt = 0;
+        FoldCursor cursor;
         if constexpr (FOLD) {
             if (a.fold.smem_prof) {
                 for (int i = tid; i < 2 * a.fold.nbins; i += blockDim.x)
@@ -652,8 +621,7 @@ __global__ void __launch_bounds__(TcShape<LOG2N>::THREADS, TcShape<LOG2N>::CTAS_
                 fw.prof_main = a.fold.part_main + (size_t)w * a.fold.nbins;
                 fw.prof_pend = a.fold.part_pend + (size_t)w * a.fold.nbins;
             }
-            sp = span_lower_bound(a.fold.span_b, a.fold.nspans, (long long)kb * M);
-            span_refill(a.fold, fw, sp, sbase, scnt);
+            cursor_init(a.fold, fw, cursor, (long long)kb * M);
         }
 
         // Gather step i of the item into operand buffer `op`: Z = X[kg + b -
@@ -854,20 +822,20 @@ __global__ void __launch_bounds__(TcShape<LOG2N>::THREADS, TcShape<LOG2N>::CTAS_
                 // detected in the item's scale; its partial profiles are
                 // rescaled once at the end of the item (the scale is a power
                 // of two, fixed for the item)
-                // sample t = t0 + N2 u at iswz(t) (kIbufSwizzled): adding
-                // N2 u = 128 u leaves the swizzle bits alone; adding 64 u
-                // flips their upper bit with u's parity
+                // sample t = t0 + N2 u at ipad(t) (kIbufPadded), N2 a multiple
+                // of 32
                 float *ib = reinterpret_cast<float *>(op);
                 const int t0 = ob * M + 16 * N2 * oh + om2;
-                const int e0 = iswz(t0), e1 = N2 == 64 ? iswz(t0 + 64) - 64 : e0;
+                const int e0 = ipad(t0);
+                constexpr int STR = N2 + N2 / 32;
                 if (a.fold.detect) {
 #pragma unroll
                     for (int u = 0; u < 16; ++u)
-                        ib[((u & 1) ? e1 : e0) + N2 * u] = sqrtf(yr[u] * yr[u] + yi[u] * yi[u]);
+                        ib[e0 + STR * u] = sqrtf(yr[u] * yr[u] + yi[u] * yi[u]);
                 } else {
 #pragma unroll
                     for (int u = 0; u < 16; ++u)
-                        ib[((u & 1) ? e1 : e0) + N2 * u] = yr[u] * yr[u] + yi[u] * yi[u];
+                        ib[e0 + STR * u] = yr[u] * yr[u] + yi[u] * yi[u];
                 }
             }
         };
@@ -919,21 +887,10 @@ __global__ void __launch_bounds__(TcShape<LOG2N>::THREADS, TcShape<LOG2N>::CTAS_
                 outputs(i, sm + cur);
                 tc_fence_before();
                 if constexpr (FOLD) {
-                    // the step's intensities are contiguous: one pass when one
-                    // period span holds them, else unit by unit (a unit: one
-                    // block at 4096 and 8192, half of the block at 16384)
-                    constexpr int FU = BPS == 2 ? M : M / 2;
                     const int k = kb + BPS * i;
-                    const bool second = BPS == 1 || k + 1 < ke;
-                    const float *ib0 = reinterpret_cast<const float *>(sm + cur);
                     __syncthreads();
-                    if (!(second && fold_pair<kIbufSwizzled>(a.fold, fw, ib0, k * M, FU, sp, sbase, scnt))) {
-                        fold_block<kIbufSwizzled>(a.fold, fw, ib0, k * M, FU, sp, sbase, scnt);
-                        if (second) {
-                            __syncthreads();
-                            fold_block<kIbufSwizzled>(a.fold, fw, ib0 + FU, k * M + FU, FU, sp, sbase, scnt);
-                        }
-                    }
+                    fold_block<kIbufPadded>(a.fold, fw, reinterpret_cast<const float *>(sm + cur), k * M,
+                                            min(ke - k, BPS) * M, cursor, 160 * (i & 15));
                 }
                 if (more) {
                     if (!wait_gemm(tid, barA, phA, wlim)) {
@@ -1125,8 +1082,6 @@ cudaError_t launch_tc_t(bool bf16, bool series, bool fold, const DedispArgs &a, 
 
 bool tc_supported(int log2n) { return log2n >= kLog2NMin && log2n <= kLog2NMax; }
 
-int tc_threads(int log2n) { return log2n == 12 ? TcShape<12>::THREADS : TcShape<13>::THREADS; }
-
 int tc_blocks_per_step(int log2n) { return log2n == 14 ? TcShape<14>::BPS : TcShape<12>::BPS; }
 
 size_t tc_smem_base(int log2n)
@@ -1162,7 +1117,7 @@ cudaError_t launch_tc_dedisp(int log2n, bool bf16, bool series, bool fold, const
     if (!a.status || !tc_supported(log2n))
         return cudaErrorInvalidValue;
     const NoBatch none{};
-    const size_t fs = fold ? fold_smem_bytes(a.fold.nbins, a.fold.span_cap, a.fold.smem_prof != 0, tc_threads(log2n))
+    const size_t fs = fold ? fold_smem_bytes(a.fold.nbins, a.fold.span_cap, a.fold.smem_prof != 0)
                            : 0;
     if (log2n == 14)
         return launch_tc_t<14, false>(bf16, series, fold, a, none, fs, grid, st);
