@@ -899,29 +899,38 @@ static msosm_status fold_prepare(msosm_dedisp *d, int sb, FoldArgs &fa)
     const int n = (int)d->spans.size();
     if (n > d->span_cap)
         return fail(MSOSM_ERR_STATE, "fold planner produced %d spans (capacity %d)", n, d->span_cap);
-    // reuse of the pinned span staging: wait for its copy two calls ago
-    CK(cudaEventSynchronize(d->ev_spans[sb]));
-    long long *h = d->span_host + (size_t)sb * 4 * d->span_cap;
-    int *hp = reinterpret_cast<int *>(h + 2 * d->span_cap);
-    for (int i = 0; i < n; ++i) {
-        h[i] = d->spans[i].a;
-        h[d->span_cap + i] = d->spans[i].b;
-        hp[i] = d->spans[i].phase0;
-        hp[d->span_cap + i] = d->spans[i].dest;
+    // reuse of the pinned span staging (long tables only): wait for its reader
+    // two calls ago
+    if (n > kSpanParam)
+        CK(cudaEventSynchronize(d->ev_spans[sb]));
+    int launched = 0;
+    CK(launch_fold_begin(d->spans.data(), n, d->span_host + (size_t)sb * 4 * d->span_cap, d->span_cap, d->span_a_d,
+                         d->span_b_d, d->span_p_d, d->span_dest_d, flush, d->acc_main, d->acc_pend,
+                         (size_t)d->D * d->nbins, d->stream, &launched));
+    d->launches += launched;
+    if (n > kSpanParam)
+        CK(cudaEventRecord(d->ev_spans[sb], d->stream));
+    const bool smem = prof_in_smem(d);
+    // the first block range that reaches into the pending period
+    fa.pend_row = d->R;
+    if (n > 0 && d->spans[n - 1].dest == 2) {
+        if (d->large) {
+            fa.pend_row = d->R - 1;  // the last rows' share of the spans
+        } else {
+            const int bps = blocks_per_step(d);
+            const long long units = (d->count + bps - 1) / bps;
+            int r = d->R - 1;
+            while (r > 0 && (long long)bps * (units * r / d->R) * (long long)d->M > d->spans[n - 1].a)
+                --r;
+            fa.pend_row = r;
+        }
     }
-    // a kernel reads the staging: copies on this stream would wait behind the
-    // next call's input copy on the copy engine, and the dedispersion kernel
-    // with them
-    CK(launch_span_upload(h, n, d->span_cap, d->span_a_d, d->span_b_d, d->span_p_d, d->span_dest_d, d->stream));
-    d->launches += n > 0 ? 1 : 0;
-    CK(cudaEventRecord(d->ev_spans[sb], d->stream));
-    if (flush) {
-        CK(launch_fold_flush(d->acc_main, d->acc_pend, (size_t)d->D * d->nbins, d->stream));
-        d->launches += 1;
+    if (!smem && !d->large) {
+        // the kernel adds to its partial rows in memory
+        const size_t prow = (size_t)d->D * d->R * d->nbins;
+        CK(cudaMemsetAsync(d->part_main, 0, sizeof(float) * prow, d->stream));
+        CK(cudaMemsetAsync(d->part_pend, 0, sizeof(float) * prow, d->stream));
     }
-    const size_t prow = (size_t)d->D * d->R * d->nbins;
-    CK(cudaMemsetAsync(d->part_main, 0, sizeof(float) * prow, d->stream));
-    CK(cudaMemsetAsync(d->part_pend, 0, sizeof(float) * prow, d->stream));
     fa.span_a = d->span_a_d;
     fa.span_b = d->span_b_d;
     fa.span_phase0 = d->span_p_d;
@@ -932,7 +941,7 @@ static msosm_status fold_prepare(msosm_dedisp *d, int sb, FoldArgs &fa)
     fa.detect = d->detect;
     fa.part_main = d->part_main;
     fa.part_pend = d->part_pend;
-    fa.smem_prof = prof_in_smem(d) ? 1 : 0;
+    fa.smem_prof = smem ? 1 : 0;
     fa.span_cap = d->win_cap;
     fa.inv_bpt = 1.0f / (float)d->bpt;
     fa.g_shift = fold_g_shift(d->bpt);
@@ -1002,9 +1011,9 @@ static msosm_status filter_block_large(msosm_dedisp *d, const void *src, InputKi
     if (ev)
         CK(cudaEventRecord(ev->e[3], d->stream));
     if (d->fold) {
-        CK(launch_fold_series(d->lI, (long long)d->count * d->M, d->R, fa, d->grid, d->D, d->stream));
-        CK(launch_fold_reduce(d->part_main, d->part_pend, d->D, d->R, d->nbins, d->acc_main, d->acc_pend,
-                              d->stream));
+        CK(launch_fold_direct(d->lI, (long long)d->count * d->M, d->R, fa, d->D, d->stream));
+        CK(launch_fold_reduce(d->part_main, d->part_pend, d->D, d->R, d->nbins, fa.pend_row, nullptr, d->acc_main,
+                              d->acc_pend, d->stream));
         d->launches += 2;
     }
     if (d->series)
@@ -1114,10 +1123,11 @@ static msosm_status call_begin(msosm_dedisp *d, const void *input, InputKind kin
 
 // The last part of a filter call, after the dedispersion kernel: the ordered
 // reduction of the R partial profile rows, the series' trailing element.
-static msosm_status call_end(msosm_dedisp *d, msosm_dedisp::CallEvents *ev, int R, unsigned long long launches0)
+static msosm_status call_end(msosm_dedisp *d, msosm_dedisp::CallEvents *ev, int pend_row, unsigned long long launches0)
 {
     if (d->fold) {
-        CK(launch_fold_reduce(d->part_main, d->part_pend, d->D, R, d->nbins, d->acc_main, d->acc_pend, d->stream));
+        CK(launch_fold_reduce(d->part_main, d->part_pend, d->D, d->R, d->nbins, pend_row, d->status_d, d->acc_main,
+                              d->acc_pend, d->stream));
         d->launches += 1;
     }
     if (d->series)
@@ -1160,7 +1170,7 @@ static msosm_status filter_block(msosm_dedisp *d, const void *input, InputKind k
     d->launches += 1;
     if (ev)
         CK(cudaEventRecord(ev->e[3], d->stream));
-    return call_end(d, ev, d->R, launches0);
+    return call_end(d, ev, da.fold.pend_row, launches0);
 }
 
 // ---------------------------------------------------------------------------
@@ -1366,7 +1376,7 @@ msosm_status msosm_batch_filter(msosm_batch *b, const void *const *inputs, int i
         CK(launch_tc_dedisp_batch(g.log2n, g.bf16, g.series, g.fold, *g.args, g.fold_smem, g.grid, b->stream));
         for (size_t j = 0; j < nm; ++j) {
             msosm_dedisp *d = b->h[g.members[j]];
-            msosm_status st = call_end(d, nullptr, g.R[j], l0[j]);
+            msosm_status st = call_end(d, nullptr, g.args->args[j].fold.pend_row, l0[j]);
             if (st != MSOSM_OK)
                 return st;
         }
@@ -1486,16 +1496,7 @@ msosm_status msosm_dedisp_fold_init(msosm_dedisp *d, float period, float fs, uns
             return cuda_fail(e, "plan_grid");
         }
     } else {
-        // the series fold: ranges of 2048-sample blocks per trial, about four
-        // thread blocks per SM over all trials
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const long long nblk = ((long long)d->count * d->M + fold_series_block() - 1) / fold_series_block();
-        long long R = (4ll * (sms > 0 ? sms : 1) + d->D - 1) / d->D;
-        R = R > nblk ? nblk : (R < 1 ? 1 : R);
-        d->R = (int)R;
-        d->grid = (int)R;
+        d->R = fold_direct_rows(d->nbins, d->bpt, d->D, d->span_cap);
     }
     d->fold = false;
     size_t &tot = d->device_bytes;
@@ -1645,7 +1646,7 @@ msosm_status msosm_dedisp_get_timing(msosm_dedisp *d, msosm_timing *t)
 
 struct msosm_fold {
     unsigned long size = 0, ps = 0;
-    int nbins = 0, bpt = 1, span_cap = 0, win_cap = 64, R = 1, grid = 1;
+    int nbins = 0, bpt = 1, span_cap = 0, R = 1;
     double out_scale = 1.0;
     float period = 0.f, fs = 0.f;
     FoldPlanner *planner = nullptr;
@@ -1707,18 +1708,7 @@ msosm_status msosm_fold_create(float period, float fs, unsigned long size, unsig
     f->bpt = nb == f->ps ? 1 : (int)(f->ps / nb);
     f->out_scale = nb == f->ps ? 1.0 : 1.0 / (double)f->bpt;
     f->span_cap = (int)(size / f->ps) + 8;
-    f->win_cap = (int)((unsigned long)fold_series_block() / f->ps) + 4;
-    if (f->win_cap < 64)
-        f->win_cap = 64;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long blocks = ((long long)size + fold_series_block() - 1) / fold_series_block();
-    long long R = 4ll * (sms > 0 ? sms : 1);
-    if (R > blocks)
-        R = blocks;
-    f->R = (int)(R < 1 ? 1 : R);
-    f->grid = f->R;
+    f->R = fold_direct_rows(f->nbins, f->bpt, 1, f->span_cap);
     size_t tot = 0;
 #define CKF(call)                                                                                      \
     do {                                                                                               \
@@ -1853,20 +1843,9 @@ msosm_status msosm_fold_data(msosm_fold *f)
     const int n = (int)f->spans.size();
     if (n > f->span_cap)
         return fail(MSOSM_ERR_STATE, "fold planner produced %d spans (capacity %d)", n, f->span_cap);
-    long long *h = f->span_host;
-    int *hp = reinterpret_cast<int *>(h + 2 * f->span_cap);
-    for (int i = 0; i < n; ++i) {
-        h[i] = f->spans[i].a;
-        h[f->span_cap + i] = f->spans[i].b;
-        hp[i] = f->spans[i].phase0;
-        hp[f->span_cap + i] = f->spans[i].dest;
-    }
-    // read by a kernel, not copied: see fold_prepare
-    CK(launch_span_upload(h, n, f->span_cap, f->span_a, f->span_b, f->span_p, f->span_dest, f->stream));
-    if (flush)
-        CK(launch_fold_flush(f->acc_main, f->acc_pend, (size_t)f->nbins, f->stream));
-    CK(cudaMemsetAsync(f->part_main, 0, sizeof(float) * f->R * f->nbins, f->stream));
-    CK(cudaMemsetAsync(f->part_pend, 0, sizeof(float) * f->R * f->nbins, f->stream));
+    int launched = 0;
+    CK(launch_fold_begin(f->spans.data(), n, f->span_host, f->span_cap, f->span_a, f->span_b, f->span_p, f->span_dest,
+                         flush, f->acc_main, f->acc_pend, (size_t)f->nbins, f->stream, &launched));
     FoldArgs a;
     a.span_a = f->span_a;
     a.span_b = f->span_b;
@@ -1878,14 +1857,17 @@ msosm_status msosm_fold_data(msosm_fold *f)
     a.detect = 0;
     a.part_main = f->part_main;
     a.part_pend = f->part_pend;
-    a.smem_prof = f->nbins <= kMaxSmemBins ? 1 : 0;
-    a.span_cap = f->win_cap;
+    a.smem_prof = 0;
+    a.span_cap = 0;
     a.inv_bpt = 1.0f / (float)f->bpt;
-    a.g_shift = fold_g_shift(f->bpt);
-    CK(launch_fold_series(f->I, (long long)f->size, f->R, a, f->grid, 1, f->stream));
-    CK(launch_fold_reduce(f->part_main, f->part_pend, 1, f->R, f->nbins, f->acc_main, f->acc_pend, f->stream));
-    // the pinned span staging is reused by the next call
-    CK(cudaStreamSynchronize(f->stream));
+    a.g_shift = 0;
+    a.pend_row = n > 0 && f->spans[n - 1].dest == 2 ? f->R - 1 : f->R;
+    CK(launch_fold_direct(f->I, (long long)f->size, f->R, a, 1, f->stream));
+    CK(launch_fold_reduce(f->part_main, f->part_pend, 1, f->R, f->nbins, a.pend_row, nullptr, f->acc_main, f->acc_pend,
+                          f->stream));
+    // the pinned span staging (long tables only) is reused by the next call
+    if (n > kSpanParam)
+        CK(cudaStreamSynchronize(f->stream));
     return MSOSM_OK;
 }
 

@@ -19,7 +19,6 @@
 // each trial gathers X[k - delay[b]][b] * H[b] directly.
 #include "chirp.cuh"
 #include "fft_smem.cuh"
-#include "fold_dev.cuh"
 #include "kernels.hpp"
 #include "tc_layout.hpp"
 
@@ -120,49 +119,62 @@ __global__ void intensity_kernel(const float2 *__restrict__ a, const float2 *__r
     }
 }
 
-// Fold n intensities (one chunk of the stream) into per-work-item partial
-// rows with the same span machinery as the fused kernel: work item w covers
-// blocks [n_blocks*w/R, n_blocks*(w+1)/R) of kFoldBlock samples.
-constexpr int kFoldBlock = 2048;
-
-__global__ void __launch_bounds__(256) fold_series_kernel(const float *__restrict__ I, long long n, int R, FoldArgs f)
+// Fold the intensities of a chunk straight from memory: a group of G = 2^g_shift
+// lanes per output bin adds the bin's samples of every span of row r's share
+// [nspans r / R, nspans (r + 1) / R) and writes them to partial row r (the main
+// and the pending sums); trial d = blockIdx.z folds I[d n ...] into rows r D + d.
+// Bound by latency: a lane's loads are independent, and blocks and rows are
+// cut so that about 1200 blocks share the chunk (fold_direct_rows).  At 84
+// periods of 49600 samples and 1024 bins the staged form (2048 samples to
+// shared memory, then folded by the block, 592 rows) took 26 us.
+__global__ void __launch_bounds__(256) fold_direct_kernel(const float *__restrict__ I, long long n, FoldArgs f)
 {
-    // trial blockIdx.y folds I[d*n ...] into partial rows w*gridDim.y + d
-    const int d = blockIdx.y, D = gridDim.y;
+    const int r = blockIdx.y, R = gridDim.y, d = blockIdx.z, D = gridDim.z;
     I += (size_t)d * n;
-    extern __shared__ float2 smem[];
-    float *ibuf = reinterpret_cast<float *>(smem);
-    FoldSmem fw;
-    fold_smem_layout(fw, ibuf + ibuf_floats(kFoldBlock), f);
-    const long long nblk = (n + kFoldBlock - 1) / kFoldBlock;
-    for (int w = blockIdx.x; w < R; w += gridDim.x) {
-        const long long kb = nblk * w / R, ke = nblk * (w + 1) / R;
-        if (f.smem_prof) {
-            for (int i = threadIdx.x; i < 2 * f.nbins; i += blockDim.x)
-                fw.prof_main[i] = 0.f;
-        } else {
-            fw.prof_main = f.part_main + ((size_t)w * D + d) * f.nbins;
-            fw.prof_pend = f.part_pend + ((size_t)w * D + d) * f.nbins;
-        }
-        FoldCursor cur;
-        cursor_init(f, fw, cur, kb * kFoldBlock);
-        for (long long k = kb; k < ke; ++k) {
-            const int t0 = (int)(k * kFoldBlock);
-            for (int t = threadIdx.x; t < kFoldBlock; t += blockDim.x)
-                ibuf[ipad(t)] = (long long)t0 + t < n ? I[t0 + t] : 0.f;
-            __syncthreads();
-            fold_block<kIbufPadded>(f, fw, ibuf, t0, kFoldBlock, cur);
-            __syncthreads();
-        }
-        if (f.smem_prof) {
-            float *gm = f.part_main + ((size_t)w * D + d) * f.nbins;
-            float *gp = f.part_pend + ((size_t)w * D + d) * f.nbins;
-            for (int i = threadIdx.x; i < f.nbins; i += blockDim.x) {
-                gm[i] = fw.prof_main[i];
-                gp[i] = fw.prof_pend[i];
+    const int G = 1 << f.g_shift, l = threadIdx.x & (G - 1);
+    const int bin = (int)blockIdx.x * (256 >> f.g_shift) + (int)(threadIdx.x >> f.g_shift);
+    const int s0 = (int)((long long)f.nspans * r / R), s1 = (int)((long long)f.nspans * (r + 1) / R);
+    float main = 0.f, pend = 0.f;
+    if (bin < f.nbins) {
+        const long long p0 = (long long)bin * f.bpt;
+        for (int s = s0; s < s1; ++s) {
+            const int dest = f.span_dest[s];
+            if (dest == 0)
+                continue;
+            const long long a = f.span_a[s], ph = f.span_phase0[s], len = f.span_b[s] - a;
+            const long long lo = p0 > ph ? p0 : ph, hi = p0 + f.bpt < ph + len ? p0 + f.bpt : ph + len;
+            const float *src = I + (a - ph) + lo;  // (only read below hi)
+            const int m = hi > lo ? (int)(hi - lo) : 0;
+            float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+            int p = l;
+            for (; p + 3 * G < m; p += 4 * G) {
+                a0 += src[p];
+                a1 += src[p + G];
+                a2 += src[p + 2 * G];
+                a3 += src[p + 3 * G];
             }
+            if (p < m)
+                a0 += src[p];
+            if (p + G < m)
+                a1 += src[p + G];
+            if (p + 2 * G < m)
+                a2 += src[p + 2 * G];
+            const float sum = (a0 + a1) + (a2 + a3);
+            if (dest == 1)
+                main += sum;
+            else
+                pend += sum;
         }
-        __syncthreads();
+    }
+    for (int o = G >> 1; o > 0; o >>= 1) {
+        main += __shfl_xor_sync(0xffffffffu, main, o);
+        pend += __shfl_xor_sync(0xffffffffu, pend, o);
+    }
+    if (bin < f.nbins && l == 0) {
+        const size_t at = ((size_t)r * D + d) * f.nbins + bin;
+        f.part_main[at] = main;
+        if (r >= f.pend_row)
+            f.part_pend[at] = pend;
     }
 }
 
@@ -229,30 +241,34 @@ __global__ void __launch_bounds__(FftShape<LOG2N>::T) design_kernel(DesignArgs a
 
 // Sum of the R partial rows of every (trial, bin), in double and in a fixed
 // order: G groups of rows (group g: rows g, g + G, ...) are summed by G
-// threads, then thread g = 0 adds the G group sums in group order.  A thread
-// block covers 32 consecutive (trial, bin) indices x G groups; row r of index
-// i sits at r * D * nbins + i, so a warp reads 128 contiguous bytes of a row.
+// threads, then thread g = 0 adds the G group sums in group order.  The
+// pending rows before pend_row hold nothing.  After a timed-out kernel (status
+// set) the rows are incomplete and nothing is added.
+// A thread block covers 32 consecutive (trial, bin) indices x G groups; row r
+// of index i sits at r * D * nbins + i, so a warp reads 128 contiguous bytes of
+// a row.
 template <int G>
 __global__ void __launch_bounds__(32 * G) fold_reduce_kernel(const float *__restrict__ pm,
-                                                             const float *__restrict__ pp, int D, int R, int nbins,
-                                                             double *am, double *ap)
+                                                             const float *__restrict__ pp, long long n, int R,
+                                                             int pend_row, const int *__restrict__ status, double *am,
+                                                             double *ap)
 {
     __shared__ double part[2][G][32];
     const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
-    const long long n = (long long)D * nbins;
     const long long i = (long long)blockIdx.x * 32 + lane;
+    const bool skip = status && *status != 0;
     double sm = 0.0, sp = 0.0;
-    if (i < n) {
-        for (int r = g; r < R; r += G) {
-            const size_t row = (size_t)r * (size_t)n + (size_t)i;
-            sm += (double)pm[row];
-            sp += (double)pp[row];
-        }
+    if (i < n && !skip) {
+#pragma unroll 4
+        for (int r = g; r < R; r += G)
+            sm += (double)pm[(size_t)r * (size_t)n + (size_t)i];
+        for (int r = pend_row + g; r < R; r += G)
+            sp += (double)pp[(size_t)r * (size_t)n + (size_t)i];
     }
     part[0][g][lane] = sm;
     part[1][g][lane] = sp;
     __syncthreads();
-    if (g == 0 && i < n) {
+    if (g == 0 && i < n && !skip) {
         double a = 0.0, b = 0.0;
 #pragma unroll
         for (int k = 0; k < G; ++k) {
@@ -262,6 +278,53 @@ __global__ void __launch_bounds__(32 * G) fold_reduce_kernel(const float *__rest
         am[i] += a;
         ap[i] += b;
     }
+}
+
+// The same for many (trial, bin) indices, four to a lane as one 16-byte read
+// (n a multiple of 4), eight groups of rows: 128 trials x 1024 bins x 16 rows,
+// 8.4 MB, at the memory's rate (63 us in the form above with the pending rows
+// read as well).
+__global__ void __launch_bounds__(256) fold_reduce4_kernel(const float4 *__restrict__ pm,
+                                                           const float4 *__restrict__ pp, long long n4, int R,
+                                                           int pend_row, const int *__restrict__ status,
+                                                           double *__restrict__ am, double *__restrict__ ap)
+{
+    constexpr int G = 8;
+    __shared__ double part[G][32][4];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const long long i = (long long)blockIdx.x * 32 + lane;
+    if (status && *status != 0)
+        return;
+    auto sum = [&](const float4 *rows, int r0, double *acc) {
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+        if (i < n4)
+#pragma unroll 4
+            for (int r = r0 + g; r < R; r += G) {
+                const float4 v = rows[(size_t)r * (size_t)n4 + (size_t)i];
+                s[0] += (double)v.x;
+                s[1] += (double)v.y;
+                s[2] += (double)v.z;
+                s[3] += (double)v.w;
+            }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            part[g][lane][k] = s[k];
+        __syncthreads();
+        // 128 threads add the groups, one value each
+        const int t = threadIdx.x;
+        const long long at = (long long)blockIdx.x * 128 + t;
+        if (t < 128 && at < 4 * n4) {
+            double a = 0.0;
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+                a += part[k][t >> 2][t & 3];
+            acc[at] += a;
+        }
+    };
+    sum(pm, 0, am);
+    if (pend_row < R)  // uniform
+        sum(pp, pend_row, ap);
 }
 
 __global__ void fold_flush_kernel(double *am, double *ap, size_t n)
@@ -390,30 +453,31 @@ cudaError_t launch_design(int log2n, const DesignArgs &a, cudaStream_t st)
 
 static unsigned int blocks_for(size_t n, unsigned int t) { return (unsigned int)((n + t - 1) / t); }
 
-cudaError_t launch_fold_reduce(const float *pm, const float *pp, int D, int R, int nbins, double *am,
-                               double *ap, cudaStream_t st)
+cudaError_t launch_fold_reduce(const float *pm, const float *pp, int D, int R, int nbins, int pend_row,
+                               const int *status, double *am, double *ap, cudaStream_t st)
 {
-    const size_t n = (size_t)D * nbins;
-    const unsigned int blocks = blocks_for(n, 32);
+    const long long n = (long long)D * nbins;
+    // from 16384 values on, 128 blocks of the 16-byte form have work enough
+    if (n >= 16384 && n % 4 == 0) {
+        fold_reduce4_kernel<<<blocks_for((size_t)n / 4, 32), 256, 0, st>>>(
+            reinterpret_cast<const float4 *>(pm), reinterpret_cast<const float4 *>(pp), n / 4, R, pend_row, status, am,
+            ap);
+        return cudaGetLastError();
+    }
+    const unsigned int blocks = blocks_for((size_t)n, 32);
     // row groups: the largest power of two <= min(R, 32)
     if (R >= 32)
-        fold_reduce_kernel<32><<<blocks, 32 * 32, 0, st>>>(pm, pp, D, R, nbins, am, ap);
+        fold_reduce_kernel<32><<<blocks, 32 * 32, 0, st>>>(pm, pp, n, R, pend_row, status, am, ap);
     else if (R >= 16)
-        fold_reduce_kernel<16><<<blocks, 32 * 16, 0, st>>>(pm, pp, D, R, nbins, am, ap);
+        fold_reduce_kernel<16><<<blocks, 32 * 16, 0, st>>>(pm, pp, n, R, pend_row, status, am, ap);
     else if (R >= 8)
-        fold_reduce_kernel<8><<<blocks, 32 * 8, 0, st>>>(pm, pp, D, R, nbins, am, ap);
+        fold_reduce_kernel<8><<<blocks, 32 * 8, 0, st>>>(pm, pp, n, R, pend_row, status, am, ap);
     else if (R >= 4)
-        fold_reduce_kernel<4><<<blocks, 32 * 4, 0, st>>>(pm, pp, D, R, nbins, am, ap);
+        fold_reduce_kernel<4><<<blocks, 32 * 4, 0, st>>>(pm, pp, n, R, pend_row, status, am, ap);
     else if (R >= 2)
-        fold_reduce_kernel<2><<<blocks, 32 * 2, 0, st>>>(pm, pp, D, R, nbins, am, ap);
+        fold_reduce_kernel<2><<<blocks, 32 * 2, 0, st>>>(pm, pp, n, R, pend_row, status, am, ap);
     else
-        fold_reduce_kernel<1><<<blocks, 32, 0, st>>>(pm, pp, D, R, nbins, am, ap);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_fold_flush(double *am, double *ap, size_t n, cudaStream_t st)
-{
-    fold_flush_kernel<<<blocks_for(n, 256), 256, 0, st>>>(am, ap, n);
+        fold_reduce_kernel<1><<<blocks, 32, 0, st>>>(pm, pp, n, R, pend_row, status, am, ap);
     return cudaGetLastError();
 }
 
@@ -432,18 +496,78 @@ __global__ void span_upload_kernel(const long long *__restrict__ h, int n, int c
     }
 }
 
-cudaError_t launch_span_upload(const long long *host, int n, int cap, long long *a, long long *b, int *phase0,
-                               int *dest, cudaStream_t st)
+// The call's spans as a launch parameter, written to the device arrays, and
+// (flush) the pending period's accumulator moved to the main one.
+struct SpanTable {
+    int n;
+    int phase0[kSpanParam], dest[kSpanParam];
+    long long a[kSpanParam], b[kSpanParam];
+};
+
+__global__ void __launch_bounds__(256) fold_begin_kernel(const __grid_constant__ SpanTable t, long long *__restrict__ a,
+                                                         long long *__restrict__ b, int *__restrict__ p,
+                                                         int *__restrict__ dest, double *am, double *ap, size_t n)
 {
-    if (n <= 0)
-        return cudaSuccess;
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < (size_t)t.n) {
+        a[i] = t.a[i];
+        b[i] = t.b[i];
+        p[i] = t.phase0[i];
+        dest[i] = t.dest[i];
+    }
+    if (i < n) {
+        am[i] += ap[i];
+        ap[i] = 0.0;
+    }
+}
+
+// Up to kSpanParam spans travel as the launch's parameter; more are read from
+// their pinned staging (which costs a bus round trip, 6 us against 2).
+cudaError_t launch_fold_begin(const FoldSpan *spans, int n, long long *host, int cap, long long *a, long long *b,
+                              int *phase0, int *dest, bool flush, double *acc_main, double *acc_pend, size_t nacc,
+                              cudaStream_t st, int *launches)
+{
+    *launches = 0;
+    if (n <= kSpanParam) {
+        if (n == 0 && !flush)
+            return cudaSuccess;
+        SpanTable t;
+        t.n = n;
+        for (int i = 0; i < n; ++i) {
+            t.a[i] = spans[i].a;
+            t.b[i] = spans[i].b;
+            t.phase0[i] = spans[i].phase0;
+            t.dest[i] = spans[i].dest;
+        }
+        const size_t work = flush ? (nacc > (size_t)n ? nacc : (size_t)n) : (size_t)n;
+        *launches = 1;
+        fold_begin_kernel<<<blocks_for(work, 256), 256, 0, st>>>(t, a, b, phase0, dest, acc_main, acc_pend,
+                                                                 flush ? nacc : 0);
+        return cudaGetLastError();
+    }
+    int *hp = reinterpret_cast<int *>(host + 2 * (size_t)cap);
+    for (int i = 0; i < n; ++i) {
+        host[i] = spans[i].a;
+        host[cap + i] = spans[i].b;
+        hp[i] = spans[i].phase0;
+        hp[cap + i] = spans[i].dest;
+    }
+    // a kernel reads the staging: copies on this stream would wait behind the
+    // next call's input copy on the copy engine, and the dedispersion kernel
+    // with them
     void *hd = nullptr;
-    cudaError_t e = cudaHostGetDevicePointer(&hd, const_cast<long long *>(host), 0);
+    cudaError_t e = cudaHostGetDevicePointer(&hd, host, 0);
     if (e != cudaSuccess)
         return e;
     const unsigned int g = blocks_for((size_t)n, 256) < 64 ? blocks_for((size_t)n, 256) : 64;
+    *launches = 1;
     span_upload_kernel<<<g, 256, 0, st>>>(static_cast<const long long *>(hd), n, cap, a, b, phase0, dest);
-    return cudaGetLastError();
+    if ((e = cudaGetLastError()) == cudaSuccess && flush) {
+        *launches = 2;
+        fold_flush_kernel<<<blocks_for(nacc, 256), 256, 0, st>>>(acc_main, acc_pend, nacc);
+        e = cudaGetLastError();
+    }
+    return e;
 }
 
 cudaError_t launch_fold_readout(const double *am, size_t n, double scale, float *out, cudaStream_t st)
@@ -458,17 +582,35 @@ cudaError_t launch_intensity(const float2 *a, const float2 *b, float *out, size_
     return cudaGetLastError();
 }
 
-int fold_series_block() { return kFoldBlock; }
-
-cudaError_t launch_fold_series(const float *I, long long n, int R, const FoldArgs &f, int grid, int trials,
-                               cudaStream_t st)
+// lanes per bin of the direct fold: about eight samples each, so that a warp
+// reads runs of memory
+static int direct_g_shift(int bpt)
 {
-    const size_t sm =
-        ibuf_floats(kFoldBlock) * sizeof(float) + fold_smem_bytes(f.nbins, f.span_cap, f.smem_prof != 0);
-    cudaError_t e = set_smem(fold_series_kernel, sm);
-    if (e != cudaSuccess)
-        return e;
-    fold_series_kernel<<<dim3((unsigned)grid, (unsigned)trials), 256, sm, st>>>(I, n, R, f);
+    int g = 0;
+    while (g < 5 && (8 << g) < bpt)
+        ++g;
+    return g;
+}
+
+static int direct_tiles(int nbins, int bpt)
+{
+    const int per = 256 >> direct_g_shift(bpt);
+    return (nbins + per - 1) / per;
+}
+
+int fold_direct_rows(int nbins, int bpt, int trials, int max_spans)
+{
+    const long long tiles = (long long)direct_tiles(nbins, bpt) * trials;
+    const long long R = 1200 / tiles;
+    return (int)(R < 1 ? 1 : (R > max_spans ? max_spans : R));
+}
+
+cudaError_t launch_fold_direct(const float *I, long long n, int R, const FoldArgs &args, int trials, cudaStream_t st)
+{
+    FoldArgs f = args;
+    f.g_shift = direct_g_shift(f.bpt);
+    fold_direct_kernel<<<dim3((unsigned)direct_tiles(f.nbins, f.bpt), (unsigned)R, (unsigned)trials), 256, 0, st>>>(I, n,
+                                                                                                                   f);
     return cudaGetLastError();
 }
 

@@ -39,6 +39,7 @@ struct FoldArgs {
     int span_cap;   // spans held in the shared-memory window (refilled as the fold goes on)
     float inv_bpt;  // 1/bpt, for the exact-corrected division
     int g_shift;    // log2 of the lanes summing one bin (fold_g_shift)
+    int pend_row;   // block ranges (rows) before this one hold no pending samples: not written, not read
 };
 
 // log2 of the lanes that sum one bin in the fold: the smallest power of two
@@ -129,23 +130,27 @@ size_t dedisp_smem(int log2n, bool fold, size_t fold_smem);
 size_t dedisp_smem_share(int log2n);
 cudaError_t launch_design(int log2n, const DesignArgs &a, cudaStream_t st);
 
-cudaError_t launch_fold_reduce(const float *part_main, const float *part_pend, int D, int R, int nbins,
-                               double *acc_main, double *acc_pend, cudaStream_t st);
-cudaError_t launch_fold_flush(double *acc_main, double *acc_pend, size_t n, cudaStream_t st);
-// The n fold spans of a call from their pinned host staging (a, b: long long
-// [cap] each, then phase0, dest: int [cap] each), read by a kernel over the
-// bus, into the device span arrays
-cudaError_t launch_span_upload(const long long *host, int n, int cap, long long *a, long long *b, int *phase0,
-                               int *dest, cudaStream_t st);
+// sums of the R partial rows onto the accumulators; status (may be null) of a
+// kernel that may have timed out
+cudaError_t launch_fold_reduce(const float *part_main, const float *part_pend, int D, int R, int nbins, int pend_row,
+                               const int *status, double *acc_main, double *acc_pend, cudaStream_t st);
+// The n fold spans of a call into the device span arrays, and with flush the
+// pending accumulator onto the main one.  More than kSpanParam spans go
+// through their pinned host staging (a, b: long long [cap] each, then phase0,
+// dest: int [cap] each), which must be free.
+constexpr int kSpanParam = 128;
+cudaError_t launch_fold_begin(const FoldSpan *spans, int n, long long *host, int cap, long long *a, long long *b,
+                              int *phase0, int *dest, bool flush, double *acc_main, double *acc_pend, size_t nacc,
+                              cudaStream_t st, int *launches);
 cudaError_t launch_fold_readout(const double *acc_main, size_t n, double scale, float *out,
                                 cudaStream_t st);
 cudaError_t launch_encode_u16(const float2 *src, uint32_t *dst, size_t n, cudaStream_t st);
 // sqrt(|a|^2 + |b|^2) (b may be null)
 cudaError_t launch_intensity(const float2 *a, const float2 *b, float *out, size_t n, cudaStream_t st);
-// fold n intensities into R partial rows (fold.part_main/part_pend [R][nbins])
-int fold_series_block();
-cudaError_t launch_fold_series(const float *I, long long n, int R, const FoldArgs &f, int grid, int trials,
-                               cudaStream_t st);
+// fold n intensities of each trial into R partial rows per trial (fold.part_main / part_pend
+// [R][trials][nbins]); the rows to use for at most max_spans spans a call
+int fold_direct_rows(int nbins, int bpt, int trials, int max_spans);
+cudaError_t launch_fold_direct(const float *I, long long n, int R, const FoldArgs &f, int trials, cudaStream_t st);
 
 // ---- tensor-core (tcgen05) dedispersion, 4096-, 8192- and 16384-point transforms (tc_dedisp.cu)
 bool tc_supported(int log2n);

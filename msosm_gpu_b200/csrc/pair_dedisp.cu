@@ -360,7 +360,8 @@ __global__ void __launch_bounds__(PairShape<LOG2N>::THREADS, PairShape<LOG2N>::C
                 float *gp = a.fold.part_pend + (size_t)w * a.fold.nbins;
                 for (int i = tid; i < a.fold.nbins; i += P::THREADS) {
                     gm[i] = fw.prof_main[i];
-                    gp[i] = fw.prof_pend[i];
+                    if (rr >= a.fold.pend_row)
+                        gp[i] = fw.prof_pend[i];
                 }
             }
         }

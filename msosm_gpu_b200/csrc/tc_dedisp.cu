@@ -947,7 +947,8 @@ __global__ void __launch_bounds__(TcShape<LOG2N>::THREADS, TcShape<LOG2N>::CTAS_
             if (a.fold.smem_prof) {
                 for (int i = tid; i < a.fold.nbins; i += blockDim.x) {
                     gm[i] = fw.prof_main[i] * back;
-                    gp[i] = fw.prof_pend[i] * back;
+                    if (rr >= a.fold.pend_row)
+                        gp[i] = fw.prof_pend[i] * back;
                 }
             } else {
                 for (int i = tid; i < a.fold.nbins; i += blockDim.x) {
