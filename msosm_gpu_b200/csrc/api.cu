@@ -978,8 +978,12 @@ static msosm_status filter_block_large(msosm_dedisp *d, const void *src, InputKi
     ra.N = N;
     ra.log2n = d->log2n;
     ra.tw2 = d->tw2f;
-    CK(launch_large_row(d->log2n2, 0, ra, 1 << d->log2n1, d->count, 1, d->stream));
-    d->launches += 2;
+    // one trial without block delays: both row passes in one, after the fold's
+    // preparation; nothing later reads its spectra
+    const bool one_row_pass = d->D == 1 && d->max_delay == 0;
+    if (!one_row_pass)
+        CK(launch_large_row(d->log2n2, 0, ra, 1 << d->log2n1, d->count, 1, d->stream));
+    d->launches += one_row_pass ? 1 : 2;
     CK(cudaEventRecord(d->ev_consumed[sb], d->stream));
     if (ev)
         CK(cudaEventRecord(ev->e[1], d->stream));
@@ -994,8 +998,12 @@ static msosm_status filter_block_large(msosm_dedisp *d, const void *src, InputKi
     ra.out = d->lB;
     ra.H = d->H;
     ra.delays = d->delays_d;
-    ra.tw2 = d->tw2i;
-    CK(launch_large_row(d->log2n2, 1, ra, 1 << d->log2n1, d->count, d->D, d->stream));
+    if (one_row_pass) {
+        ra.tw2i = d->tw2i;
+    } else {
+        ra.tw2 = d->tw2i;
+    }
+    CK(launch_large_row(d->log2n2, one_row_pass ? 3 : 1, ra, 1 << d->log2n1, d->count, d->D, d->stream));
     LargeColArgs ia{};
     ia.in = d->lB;
     ia.N = N;

@@ -206,12 +206,14 @@ struct LargeRowArgs {
     long long N;
     int log2n;
     const float2 *tw2;        // exp(sign 2 pi i e / N2)
+    const float2 *tw2i;       // mode 3: the inverse pass's table
 };
 void large_split(int log2n, int &log2n1, int &log2n2);
 bool large_supported(int log2n);
 cudaError_t launch_large_col_fwd(int log2n1, int kind, const LargeColArgs &a, int windows, cudaStream_t st);
 cudaError_t launch_large_col_inv(int log2n1, const LargeColArgs &a, int blocks, int trials, cudaStream_t st);
-// mode 0: forward row -> ring; 1: gather x H, inverse row -> B; 2: forward row -> out
+// mode 0: forward row -> ring; 1: gather x H, inverse row -> B; 2: forward row
+// -> out; 3: forward row, x H, inverse row -> B (one trial, no block delays)
 cudaError_t launch_large_row(int log2n2, int mode, const LargeRowArgs &a, int rows, int windows, int trials,
                              cudaStream_t st);
 cudaError_t launch_vec_fft(int log2n, int sign, const float2 *in, float2 *out, const float2 *tw, int count,

@@ -12,10 +12,10 @@
 // no transpose is ever made.  The inverse column pass computes only
 // n1 >= N1/2, the overlap-save half that is kept.
 //
-// Column passes run 16 columns per thread block (16 independent N1-point
-// block FFTs whose global reads and writes are 128-byte rows); row passes run
-// one N2-point block FFT per thread block.  Twiddles W_N^e come from
-// sincospif of the exact float 2e/N.
+// Column passes run 16 or 32 columns per thread block (independent N1-point
+// block FFTs whose global reads and writes are rows of 16 or 32 elements); row
+// passes run one N2-point block FFT per thread block.  Twiddles W_N^e come
+// from sincospif of the exact float 2e/N and products of two or three of them.
 #include "chirp.cuh"
 #include "fft_smem.cuh"
 #include "kernels.hpp"
@@ -26,22 +26,52 @@ namespace msosm {
 
 namespace {
 
-constexpr int kCols = 16;  // columns per thread block in the column passes
-
+// Columns per thread block in the column passes: 32 up to 128 points (128-byte
+// rows of uint16 pairs, 256-byte rows of float2), 16 above, where the buffers
+// and threads of 16 columns fill a block.
 template <int LOG2N1>
 struct ColShape {
     using F = FftShape<LOG2N1>;
-    static constexpr int STR = F::SMEM + 1;  // odd stride: 16 columns hit 16 bank pairs
-    static constexpr int THREADS = kCols * F::T;
-    static constexpr size_t SMEM_BYTES = (size_t)kCols * STR * sizeof(float2);
+    static constexpr int COLS = LOG2N1 <= 7 ? 32 : 16;
+    static constexpr int STR = F::SMEM + 1;  // odd stride: the columns hit different bank pairs
+    static constexpr int THREADS = COLS * F::T;
+    static constexpr int BLOCKS = THREADS >= 1024 ? 1 : 1024 / THREADS;  // per SM: 64 registers a thread
+    static constexpr size_t SMEM_BYTES = (size_t)COLS * STR * sizeof(float2);
 };
 
-__device__ __forceinline__ float2 twiddle_n(long long e, int log2n, float sign)
+__device__ __forceinline__ float2 twiddle_n(int e, int log2n, float sign)
 {
-    // exp(sign * 2 pi i e / N): 2e/N is exact in float for N <= 2^24
+    // exp(sign * 2 pi i e / N), 0 <= e < N: 2e/N is exact in float for N <= 2^24
     float s, c;
     sincospif(ldexpf((float)(2 * e), -log2n), &s, &c);
     return make_float2(c, sign * s);
+}
+
+// v[slot] *= W_N^(sign a k), k = j + m T the output index of the slot
+// (last_out_index: slot q R + r holds m = q + r 16/R).  Five sines and cosines and at most
+// three products per factor instead of sixteen: those, with the 64-bit
+// indices, were most of the column pass's instructions (54 us for 32 windows
+// of 2^18 points).
+template <int LOG2L>
+__device__ __forceinline__ void twiddle_outputs(float2 (&v)[16], int a, int j, int log2n, float sign)
+{
+    using F = FftShape<LOG2L>;
+    constexpr int R = F::radix(F::NST - 1), B = 16 / R;
+    const int s = a * F::T;
+    float2 b[4];
+    b[1] = twiddle_n(s, log2n, sign);
+    b[2] = cmul(b[1], b[1]);
+    b[3] = cmul(b[2], b[1]);
+    const float2 w0 = twiddle_n(a * j, log2n, sign);
+#pragma unroll
+    for (int m4 = 0; m4 < 4; ++m4) {
+        const float2 c = m4 == 0 ? w0 : cmul(w0, twiddle_n(4 * m4 * s, log2n, sign));
+#pragma unroll
+        for (int m1 = 0; m1 < 4; ++m1) {
+            const int m = 4 * m4 + m1, slot = (m % B) * R + m / B;
+            v[slot] = cmul(v[slot], m1 == 0 ? c : cmul(c, b[m1]));
+        }
+    }
 }
 
 template <int KIND>
@@ -61,41 +91,49 @@ __device__ __forceinline__ float2 load_in(const void *p, long long s)
 // indices from the previous call's history); KIND 2: a plain vector of
 // length `len` (zero beyond).  Output A[w][k1][n2] with the twiddle applied.
 template <int LOG2N1, int KIND>
-__global__ void __launch_bounds__(ColShape<LOG2N1>::THREADS) lcol_fwd_kernel(LargeColArgs a)
+__global__ void __launch_bounds__(ColShape<LOG2N1>::THREADS, ColShape<LOG2N1>::BLOCKS) lcol_fwd_kernel(LargeColArgs a)
 {
     using F = FftShape<LOG2N1>;
     using C = ColShape<LOG2N1>;
     constexpr int T1 = F::T;
     extern __shared__ float2 smem[];
-    const int c = threadIdx.x % kCols, j = threadIdx.x / kCols;
-    const long long n2 = (long long)blockIdx.x * kCols + c;
+    const int c = threadIdx.x % C::COLS, j = threadIdx.x / C::COLS;
+    const int n2 = (int)blockIdx.x * C::COLS + c;
     const int w = blockIdx.y;
-    const long long N = a.N, N2 = a.N2, M = N / 2;
+    const int N2 = (int)a.N2, M = (int)(a.N / 2);  // N <= 2^24
     float2 *buf = smem + c * C::STR;
     float2 v[16];
+    if constexpr (KIND == 2) {
 #pragma unroll
-    for (int r = 0; r < 16; ++r) {
-        const long long pos = N2 * (j + r * T1) + n2;
-        float2 x;
-        if constexpr (KIND == 2) {
-            x = pos < a.len ? reinterpret_cast<const float2 *>(a.input)[pos] : make_float2(0.f, 0.f);
-        } else {
-            const long long s = (long long)w * M + pos - M;
-            x = s < 0 ? a.hist_in[M + s] : load_in<KIND>(a.input, s);
-            if (w == a.count - 1 && pos >= M)
-                a.hist_out[pos - M] = x;
+        for (int r = 0; r < 16; ++r) {
+            const int pos = N2 * (j + r * T1) + n2;
+            v[r] = pos < a.len ? reinterpret_cast<const float2 *>(a.input)[pos] : make_float2(0.f, 0.f);
         }
-        v[r] = x;
+    } else {
+        // rows r < 8 are the window's first half (T1 rows are N1/16): the block
+        // before it, or the previous call's last one
+        const long long s0 = (long long)(w - 1) * M;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int pos = N2 * (j + r * T1) + n2;
+            v[r] = w == 0 ? a.hist_in[pos] : load_in<KIND>(a.input, s0 + pos);
+        }
+#pragma unroll
+        for (int r = 8; r < 16; ++r)
+            v[r] = load_in<KIND>(a.input, s0 + (N2 * (j + r * T1) + n2));
+        if (w == a.count - 1)
+#pragma unroll
+            for (int r = 8; r < 16; ++r)
+                a.hist_out[N2 * (j + r * T1) + n2 - M] = v[r];
     }
     dft16<-1>(v);
     stage_store<LOG2N1, 0>(v, buf, j);
     run_stages<LOG2N1, -1, false>(v, buf, buf, j, a.tw1);
-    float2 *out = a.out + (size_t)w * N;
+    twiddle_outputs<LOG2N1>(v, n2, j, a.log2n, -1.f);
+    float2 *out = a.out + (size_t)w * a.N + n2;
 #pragma unroll
-    for (int slot = 0; slot < 16; ++slot) {
-        const int k1 = last_out_index<LOG2N1>(j, slot);
-        out[(size_t)k1 * N2 + n2] = cmul(v[slot], twiddle_n(n2 * k1, a.log2n, -1.f));
-    }
+    for (int slot = 0; slot < 16; ++slot)
+        out[last_out_index<LOG2N1>(j, slot) * N2] = v[slot];
 }
 
 // Row passes (one N2-point FFT per thread block, row k1 = blockIdx.x, window
@@ -104,8 +142,11 @@ __global__ void __launch_bounds__(ColShape<LOG2N1>::THREADS) lcol_fwd_kernel(Lar
 //   MODE 1 inverse:  gather X[k - delay][k1][k2] * H[d][k1][k2] from the ring,
 //                    inverse FFT, twiddle W_N^(-n2 k1) -> B[d][w][k1][n2]
 //   MODE 2 forward:  A[w][k1][:] -> out[w][k1][:] (filter design)
+//   MODE 3 both (one trial without block delays, classical overlap-save):
+//                    A[w][k1][:] forward, x H, inverse, twiddle -> B[w][k1][n2];
+//                    the spectrum never goes to memory
 template <int LOG2N2, int MODE>
-__global__ void __launch_bounds__(FftShape<LOG2N2>::T) lrow_kernel(LargeRowArgs a)
+__global__ void __launch_bounds__(FftShape<LOG2N2>::T, FftShape<LOG2N2>::T >= 1024 ? 1 : (FftShape<LOG2N2>::T <= 64 ? 16 : 1024 / FftShape<LOG2N2>::T)) lrow_kernel(LargeRowArgs a)
 {
     using F = FftShape<LOG2N2>;
     constexpr int N2 = F::N, T2 = F::T;
@@ -121,23 +162,15 @@ __global__ void __launch_bounds__(FftShape<LOG2N2>::T) lrow_kernel(LargeRowArgs 
         const int slot_k = (int)(kg & smask);
         const float2 *__restrict__ Hd = a.H + (size_t)d * N + row;
         const uint16_t *__restrict__ dl = a.delays + (size_t)d * N + row;
+        const float2 *__restrict__ ring = a.ring + row;
 #pragma unroll
         for (int r = 0; r < 16; ++r) {
             const int k2 = j + r * T2;
             const int dly = (int)dl[k2];
             float2 x = make_float2(0.f, 0.f);
             if (kg >= dly)
-                x = a.ring[(size_t)((slot_k - dly) & smask) * N + row + k2];
+                x = ring[(size_t)((slot_k - dly) & smask) * N + k2];
             v[r] = cmul(x, Hd[k2]);
-        }
-        dft16<+1>(v);
-        stage_store<LOG2N2, 0>(v, smem, j);
-        run_stages<LOG2N2, +1, false>(v, smem, smem, j, a.tw2);
-        float2 *out = a.out + ((size_t)d * a.count + w) * N + row;
-#pragma unroll
-        for (int slot = 0; slot < 16; ++slot) {
-            const int n2 = last_out_index<LOG2N2>(j, slot);
-            out[n2] = cmul(v[slot], twiddle_n((long long)n2 * k1, a.log2n, +1.f));
         }
     } else {
         const float2 *in = a.in + (size_t)w * N + row;
@@ -147,6 +180,31 @@ __global__ void __launch_bounds__(FftShape<LOG2N2>::T) lrow_kernel(LargeRowArgs 
         dft16<-1>(v);
         stage_store<LOG2N2, 0>(v, smem, j);
         run_stages<LOG2N2, -1, false>(v, smem, smem, j, a.tw2);
+    }
+    if constexpr (MODE == 3) {
+        // the slots hold k2 = j + m T2, the inverse's inputs in another order
+        constexpr int R = F::radix(F::NST - 1), B = 16 / R;
+        const float2 *__restrict__ Hd = a.H + row + j;
+        float2 x[16];
+#pragma unroll
+        for (int m = 0; m < 16; ++m)
+            x[m] = cmul(v[(m % B) * R + m / B], Hd[m * T2]);
+#pragma unroll
+        for (int m = 0; m < 16; ++m)
+            v[m] = x[m];
+        __syncthreads();  // the forward transform's last loads
+    }
+    if constexpr (MODE == 1 || MODE == 3) {
+        dft16<+1>(v);
+        stage_store<LOG2N2, 0>(v, smem, j);
+        // (the twiddles of the two directions are conjugate tables)
+        run_stages<LOG2N2, +1, false>(v, smem, smem, j, MODE == 3 ? a.tw2i : a.tw2);
+        twiddle_outputs<LOG2N2>(v, k1, j, a.log2n, +1.f);
+        float2 *out = a.out + ((size_t)d * a.count + w) * N + row;
+#pragma unroll
+        for (int slot = 0; slot < 16; ++slot)
+            out[last_out_index<LOG2N2>(j, slot)] = v[slot];
+    } else {
         float2 *out = MODE == 0 ? a.ring + (size_t)((a.k0 + w) & (a.S - 1)) * N + row
                                 : a.out + (size_t)w * N + row;
 #pragma unroll
@@ -159,23 +217,24 @@ __global__ void __launch_bounds__(FftShape<LOG2N2>::T) lrow_kernel(LargeRowArgs 
 // t = N2*(n1 - N1/2) + n2 of block w goes to series[d][w*M + t] and/or, as
 // |y|^2 or |y|, to intensity[d][w*M + t].
 template <int LOG2N1>
-__global__ void __launch_bounds__(ColShape<LOG2N1>::THREADS) lcol_inv_kernel(LargeColArgs a)
+__global__ void __launch_bounds__(ColShape<LOG2N1>::THREADS, ColShape<LOG2N1>::BLOCKS) lcol_inv_kernel(LargeColArgs a)
 {
     using F = FftShape<LOG2N1>;
     using C = ColShape<LOG2N1>;
     constexpr int T1 = F::T, N1 = F::N;
     constexpr int RL = F::radix(F::NST - 1);
     extern __shared__ float2 smem[];
-    const int c = threadIdx.x % kCols, j = threadIdx.x / kCols;
-    const long long n2 = (long long)blockIdx.x * kCols + c;
+    const int c = threadIdx.x % C::COLS, j = threadIdx.x / C::COLS;
+    const int n2 = (int)blockIdx.x * C::COLS + c;
     const int w = blockIdx.y, d = blockIdx.z;
-    const long long N = a.N, N2 = a.N2, M = N / 2;
+    const long long N = a.N, M = N / 2;
+    const int N2 = (int)a.N2;
     float2 *buf = smem + c * C::STR;
     const float2 *in = a.in + ((size_t)d * a.count + w) * N;
     float2 v[16];
 #pragma unroll
     for (int r = 0; r < 16; ++r)
-        v[r] = in[(size_t)(j + r * T1) * N2 + n2];
+        v[r] = in[(j + r * T1) * N2 + n2];
     dft16<+1>(v);
     stage_store<LOG2N1, 0>(v, buf, j);
     run_stages<LOG2N1, +1, false>(v, buf, buf, j, a.tw1);
@@ -184,7 +243,7 @@ __global__ void __launch_bounds__(ColShape<LOG2N1>::THREADS) lcol_inv_kernel(Lar
     for (int slot = 0; slot < 16; ++slot) {
         if ((slot % RL) >= RL / 2) {
             const int n1 = last_out_index<LOG2N1>(j, slot);
-            const size_t t = (size_t)N2 * (n1 - N1 / 2) + n2;
+            const int t = N2 * (n1 - N1 / 2) + n2;
             const float2 y = v[slot];
             if (a.series)
                 a.series[base + t] = y;
@@ -289,7 +348,7 @@ template <int L1>
 cudaError_t col_fwd_t(int kind, const LargeColArgs &a, int windows, cudaStream_t st)
 {
     using C = ColShape<L1>;
-    const dim3 grid((unsigned)(a.N2 / kCols), (unsigned)windows);
+    const dim3 grid((unsigned)(a.N2 / C::COLS), (unsigned)windows);
     cudaError_t e;
     if (kind == kInputU16) {
         auto k = lcol_fwd_kernel<L1, kInputU16>;
@@ -318,7 +377,7 @@ cudaError_t col_inv_t(const LargeColArgs &a, int blocks, int trials, cudaStream_
     cudaError_t e = smem_attr(k, C::SMEM_BYTES);
     if (e != cudaSuccess)
         return e;
-    k<<<dim3((unsigned)(a.N2 / kCols), (unsigned)blocks, (unsigned)trials), C::THREADS, C::SMEM_BYTES, st>>>(a);
+    k<<<dim3((unsigned)(a.N2 / C::COLS), (unsigned)blocks, (unsigned)trials), C::THREADS, C::SMEM_BYTES, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -338,6 +397,8 @@ cudaError_t row_t(int mode, const LargeRowArgs &a, int rows, int windows, int tr
         return go(lrow_kernel<L2, 0>);
     if (mode == 1)
         return go(lrow_kernel<L2, 1>);
+    if (mode == 3)
+        return go(lrow_kernel<L2, 3>);
     return go(lrow_kernel<L2, 2>);
 }
 
@@ -357,8 +418,11 @@ cudaError_t vec_t(const float2 *in, float2 *out, const float2 *tw, int count, cu
 
 void large_split(int log2n, int &log2n1, int &log2n2)
 {
-    // N2 as large as a block FFT allows (16384), N1 >= 64 columns of 16
-    log2n2 = log2n - 6 < kMaxLog2N ? log2n - 6 : kMaxLog2N;
+    // rows of 4096 points where the columns allow it (64 <= N1 <= 1024): four
+    // row blocks per SM and as many of them as one window has rows.  With rows
+    // of 16384 points a window of 2^21 filled 128 SMs with one block each (24 us a
+    // row pass)
+    log2n2 = log2n - 6 < 12 ? log2n - 6 : (log2n - 10 > 12 ? log2n - 10 : 12);
     log2n1 = log2n - log2n2;
 }
 
