@@ -1,0 +1,71 @@
+"""Result arrays in page-locked host memory.
+
+A copy from the device into fresh pageable memory is staged by the driver and
+pays a page fault per 4 KB: 512 KB take 125 us, into page-locked memory 22 us.
+``empty`` hands out arrays over page-locked blocks; when an array and every view
+of it are gone its block goes back to a pool (at most POOL_BYTES in all, handed
+out or waiting; beyond that, and for small or very large results, the array is
+an ordinary one).  Safe to use from several threads.
+"""
+from __future__ import annotations
+
+import ctypes
+import threading
+
+import numpy as np
+
+MIN_BYTES = 32 << 10   # below, the driver's staging costs no more
+MAX_BYTES = 32 << 20
+POOL_BYTES = 128 << 20
+
+_lock = threading.RLock()  # re-entrant: an array may be collected while the pool is in use
+_free: "dict[int, list]" = {}  # block size -> addresses
+_total = 0                     # bytes of all blocks
+
+
+def _take(size: int):
+    """Address of a block of `size` bytes, or None."""
+    global _total
+    from ._abi import lib
+    with _lock:
+        if _free.get(size):
+            return _free[size].pop()
+        while _total + size > POOL_BYTES:
+            other = next((s for s, b in _free.items() if b), None)
+            if other is None:
+                return None
+            lib().msosm_host_free(ctypes.c_void_p(_free[other].pop()), 1)
+            _total -= other
+        p = ctypes.c_void_p()
+        if lib().msosm_host_alloc(size, 1, ctypes.byref(p)) != 0 or not p.value:
+            return None
+        _total += size
+        return p.value
+
+
+class _Block:
+    """Owner of a block for as long as an array refers to it."""
+
+    def __init__(self, address: int, size: int, shape, dtype):
+        self._address, self._size = address, size
+        self.__array_interface__ = {"data": (address, False), "shape": tuple(shape), "typestr": np.dtype(dtype).str,
+                                    "version": 3}
+
+    def __del__(self):
+        try:
+            with _lock:
+                _free.setdefault(self._size, []).append(self._address)
+        except Exception:  # interpreter shutdown
+            pass
+
+
+def empty(shape, dtype) -> np.ndarray:
+    """An uninitialised result array (page-locked where it pays)."""
+    shape = (int(shape),) if np.isscalar(shape) else tuple(int(s) for s in shape)
+    nbytes = int(np.prod(shape)) * np.dtype(dtype).itemsize
+    if MIN_BYTES <= nbytes <= MAX_BYTES:
+        size = 1 << (nbytes - 1).bit_length()
+        address = _take(size)
+        if address is not None:
+            return np.asarray(_Block(address, size, shape, dtype))
+    return np.empty(shape, dtype)

@@ -713,8 +713,11 @@ msosm_status msosm_dedisp_create(const float *bw, const float *dm, const float *
     CKD(cudaMemsetAsync(d->hist, 0, sizeof(float2) * 2 * M, d->stream));
     for (int i = 0; i < 2; ++i)
         CKD(dalloc((float2 **)&d->staging[i], (size_t)count * M, tot));
-    if (d->series)
+    if (d->series) {
+        // (the trailing element of the reference's layout stays zero)
         CKD(dalloc(&d->series_buf, (size_t)numDMs * count * M + 1, tot));
+        CKD(cudaMemsetAsync(d->series_buf + (size_t)numDMs * count * M, 0, sizeof(float2), d->stream));
+    }
     if (d->large)
         large_split(log2n, d->log2n1, d->log2n2);
     {
@@ -984,7 +987,8 @@ static msosm_status filter_block_large(msosm_dedisp *d, const void *src, InputKi
     if (!one_row_pass)
         CK(launch_large_row(d->log2n2, 0, ra, 1 << d->log2n1, d->count, 1, d->stream));
     d->launches += one_row_pass ? 1 : 2;
-    CK(cudaEventRecord(d->ev_consumed[sb], d->stream));
+    if (src == d->staging[sb])
+        CK(cudaEventRecord(d->ev_consumed[sb], d->stream));
     if (ev)
         CK(cudaEventRecord(ev->e[1], d->stream));
     FoldArgs fa{};
@@ -1024,8 +1028,6 @@ static msosm_status filter_block_large(msosm_dedisp *d, const void *src, InputKi
                               d->acc_pend, d->stream));
         d->launches += 2;
     }
-    if (d->series)
-        CK(cudaMemsetAsync(d->series_buf + (size_t)d->D * d->count * d->M, 0, sizeof(float2), d->stream));
     if (ev) {
         CK(cudaEventRecord(ev->e[6], d->stream));
         d->timed_launches += d->launches - launches0;
@@ -1098,7 +1100,8 @@ static msosm_status call_begin(msosm_dedisp *d, const void *input, InputKind kin
         CK(cudaEventRecord(ev->e[0], d->stream));
     CK(launch_forward(d->log2n, kind, fa, d->stream));
     d->launches += 1;
-    CK(cudaEventRecord(d->ev_consumed[sb], d->stream));
+    if (src == d->staging[sb])
+        CK(cudaEventRecord(d->ev_consumed[sb], d->stream));
     if (ev)
         CK(cudaEventRecord(ev->e[1], d->stream));
 
@@ -1130,7 +1133,7 @@ static msosm_status call_begin(msosm_dedisp *d, const void *input, InputKind kin
 }
 
 // The last part of a filter call, after the dedispersion kernel: the ordered
-// reduction of the R partial profile rows, the series' trailing element.
+// reduction of the R partial profile rows.
 static msosm_status call_end(msosm_dedisp *d, msosm_dedisp::CallEvents *ev, int pend_row, unsigned long long launches0)
 {
     if (d->fold) {
@@ -1138,8 +1141,6 @@ static msosm_status call_end(msosm_dedisp *d, msosm_dedisp::CallEvents *ev, int 
                               d->acc_pend, d->stream));
         d->launches += 1;
     }
-    if (d->series)
-        CK(cudaMemsetAsync(d->series_buf + (size_t)d->D * d->count * d->M, 0, sizeof(float2), d->stream));
     if (ev) {
         CK(cudaEventRecord(ev->e[6], d->stream));
         d->timed_launches += d->launches - launches0;

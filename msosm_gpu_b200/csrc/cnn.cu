@@ -424,7 +424,7 @@ cudaError_t launch_conv(int K, const float *in, int Cin, int L, const float *w, 
         const int cg = shape.cg, tt = shape.tt;
         const size_t sm = sizeof(float) * 2 * kCiChunk * ((size_t)conv_xw(tt) + (size_t)KK * kCoBlock * cg);
         auto k = conv_kernel<KK, BWD>;
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaError_t e = allow_smem(k, sm);
         if (e != cudaSuccess)
             return e;
         const dim3 grid(B, (Cout / kCoBlock + cg - 1) / cg, (L + kT * tt - 1) / (kT * tt));
@@ -443,7 +443,7 @@ cudaError_t launch_wgrad(int K, const float *g, int Co, const float *a, int Ci, 
         const int groups = wgrad_groups(Co, Ci, B);
         const size_t sm = sizeof(float) * kWgStages * kWgStage;
         auto k = conv_wgrad_kernel<KK>;
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaError_t e = allow_smem(k, sm);
         if (e != cudaSuccess)
             return e;
         k<<<dim3(Ci / kWgCi, (Co + kWgCo - 1) / kWgCo, groups), 128, sm, st>>>(g, Co, a, Ci, B, L, groups, part);

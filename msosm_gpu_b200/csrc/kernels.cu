@@ -22,6 +22,10 @@
 #include "kernels.hpp"
 #include "tc_layout.hpp"
 
+#include <map>
+#include <mutex>
+#include <utility>
+
 #include <cuda_runtime.h>
 
 namespace msosm {
@@ -377,10 +381,25 @@ size_t fft_smem_bytes()
     return (use_pingpong<LOG2N>() ? 2 : 1) * F::SMEM * sizeof(float2);
 }
 
-template <typename K>
-static cudaError_t set_smem(K kernel, size_t bytes)
+cudaError_t allow_smem(const void *kernel, size_t bytes, bool max_carveout)
 {
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    static std::mutex m;
+    static std::map<std::pair<const void *, int>, size_t> allowed;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess)
+        return e;
+    const std::lock_guard<std::mutex> lock(m);
+    const auto it = allowed.find({kernel, dev});
+    if (it != allowed.end() && it->second >= bytes)
+        return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess && max_carveout)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 (int)cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess)
+        allowed[{kernel, dev}] = bytes;
+    return e;
 }
 
 template <int LOG2N>
@@ -391,12 +410,12 @@ static cudaError_t forward_t(InputKind kind, const FwdArgs &a, cudaStream_t st)
     cudaError_t e;
     if (kind == kInputU16) {
         auto k = forward_kernel<LOG2N, kInputU16, PP>;
-        if ((e = set_smem(k, sm)) != cudaSuccess)
+        if ((e = allow_smem(k, sm)) != cudaSuccess)
             return e;
         k<<<a.count, FftShape<LOG2N>::T, sm, st>>>(a);
     } else {
         auto k = forward_kernel<LOG2N, kInputC64, PP>;
-        if ((e = set_smem(k, sm)) != cudaSuccess)
+        if ((e = allow_smem(k, sm)) != cudaSuccess)
             return e;
         k<<<a.count, FftShape<LOG2N>::T, sm, st>>>(a);
     }
@@ -414,7 +433,7 @@ static cudaError_t design_t(const DesignArgs &a, cudaStream_t st)
     constexpr bool PP = use_pingpong<LOG2N>();
     const size_t sm = fft_smem_bytes<LOG2N>();
     auto k = design_kernel<LOG2N, PP>;
-    cudaError_t e = set_smem(k, sm);
+    cudaError_t e = allow_smem(k, sm);
     if (e != cudaSuccess)
         return e;
     k<<<a.D, FftShape<LOG2N>::T, sm, st>>>(a);

@@ -115,6 +115,16 @@ struct DesignArgs {
 
 bool log2n_supported(int log2n);
 
+// Allows a kernel `bytes` of dynamic shared memory on the current device (and,
+// max_carveout, asks for the largest shared-memory carveout).  The attribute is
+// raised once per kernel and device and kept; any thread may ask.
+cudaError_t allow_smem(const void *kernel, size_t bytes, bool max_carveout = false);
+template <typename... A>
+cudaError_t allow_smem(void (*kernel)(A...), size_t bytes, bool max_carveout = false)
+{
+    return allow_smem(reinterpret_cast<const void *>(kernel), bytes, max_carveout);
+}
+
 // Sets the message msosm_last_error() returns on this thread.
 void set_error_message(const char *msg);
 

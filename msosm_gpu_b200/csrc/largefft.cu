@@ -313,12 +313,6 @@ __global__ void __launch_bounds__(FftShape<LOG2N>::T) vec_fft_kernel(const float
         out[off + last_out_index<LOG2N>(j, slot)] = v[slot];
 }
 
-template <typename K>
-cudaError_t smem_attr(K k, size_t bytes)
-{
-    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 unsigned int nblk(long long n, unsigned int t) { return (unsigned int)((n + t - 1) / t); }
 
 #define LDISPATCH_COL(log2n, CALL)                                                                     \
@@ -352,17 +346,17 @@ cudaError_t col_fwd_t(int kind, const LargeColArgs &a, int windows, cudaStream_t
     cudaError_t e;
     if (kind == kInputU16) {
         auto k = lcol_fwd_kernel<L1, kInputU16>;
-        if ((e = smem_attr(k, C::SMEM_BYTES)) != cudaSuccess)
+        if ((e = allow_smem(k, C::SMEM_BYTES)) != cudaSuccess)
             return e;
         k<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(a);
     } else if (kind == kInputC64) {
         auto k = lcol_fwd_kernel<L1, kInputC64>;
-        if ((e = smem_attr(k, C::SMEM_BYTES)) != cudaSuccess)
+        if ((e = allow_smem(k, C::SMEM_BYTES)) != cudaSuccess)
             return e;
         k<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(a);
     } else {
         auto k = lcol_fwd_kernel<L1, 2>;
-        if ((e = smem_attr(k, C::SMEM_BYTES)) != cudaSuccess)
+        if ((e = allow_smem(k, C::SMEM_BYTES)) != cudaSuccess)
             return e;
         k<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(a);
     }
@@ -374,7 +368,7 @@ cudaError_t col_inv_t(const LargeColArgs &a, int blocks, int trials, cudaStream_
 {
     using C = ColShape<L1>;
     auto k = lcol_inv_kernel<L1>;
-    cudaError_t e = smem_attr(k, C::SMEM_BYTES);
+    cudaError_t e = allow_smem(k, C::SMEM_BYTES);
     if (e != cudaSuccess)
         return e;
     k<<<dim3((unsigned)(a.N2 / C::COLS), (unsigned)blocks, (unsigned)trials), C::THREADS, C::SMEM_BYTES, st>>>(a);
@@ -388,7 +382,7 @@ cudaError_t row_t(int mode, const LargeRowArgs &a, int rows, int windows, int tr
     const dim3 grid((unsigned)rows, (unsigned)windows, (unsigned)trials);
     cudaError_t e;
     auto go = [&](auto k) -> cudaError_t {
-        if ((e = smem_attr(k, sm)) != cudaSuccess)
+        if ((e = allow_smem(k, sm)) != cudaSuccess)
             return e;
         k<<<grid, FftShape<L2>::T, sm, st>>>(a);
         return cudaGetLastError();
@@ -407,7 +401,7 @@ cudaError_t vec_t(const float2 *in, float2 *out, const float2 *tw, int count, cu
 {
     const size_t sm = FftShape<L>::SMEM * sizeof(float2);
     auto k = vec_fft_kernel<L, SIGN>;
-    cudaError_t e = smem_attr(k, sm);
+    cudaError_t e = allow_smem(k, sm);
     if (e != cudaSuccess)
         return e;
     k<<<count, FftShape<L>::T, sm, st>>>(in, out, tw);

@@ -407,7 +407,7 @@ cudaError_t launch_t(bool series, bool fold, const DedispArgs &a, int grid, cuda
     const size_t sm = pair_smem<LOG2N>(
         fold, fold ? fold_smem_bytes(a.fold.nbins, a.fold.span_cap, a.fold.smem_prof != 0) : 0);
     return pair_select<LOG2N>(series, fold, [&](auto k) -> cudaError_t {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaError_t e = allow_smem(k, sm);
         if (e != cudaSuccess)
             return e;
         k<<<grid, P::THREADS, sm, st>>>(a);

@@ -1093,10 +1093,7 @@ cudaError_t launch_tc_t(bool bf16, bool series, bool fold, const DedispArgs &a, 
     if (S::CTAS_PER_SM == 1 && sm * 2 <= 228u * 1024u)
         return cudaErrorInvalidConfiguration;
     return tc_select_n<LOG2N, MULTI>(bf16, series, fold, [&](auto k) -> cudaError_t {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     (int)cudaSharedmemCarveoutMaxShared);
+        const cudaError_t e = allow_smem(k, sm, true);
         if (e != cudaSuccess)
             return e;
         k<<<grid, S::THREADS, sm, st>>>(a, b);
@@ -1179,7 +1176,7 @@ cudaError_t launch_tc_probe(int step, const uint16_t *a, float *d, int *status, 
     if (step < 1 || step > 4)
         return cudaErrorInvalidValue;
     auto run = [&](auto k, size_t sm, int st_) -> cudaError_t {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        const cudaError_t e = allow_smem(k, sm);
         if (e != cudaSuccess)
             return e;
         k<<<1, kThreads, sm, st>>>(st_, a, d, status);

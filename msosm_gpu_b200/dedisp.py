@@ -12,7 +12,7 @@ from typing import Optional, Sequence
 
 import numpy as np
 
-from . import _abi
+from . import _abi, _pinned
 from ._abi import check, lib
 
 
@@ -166,11 +166,11 @@ class Dedisperser:
         elements the reference layout (trailing zero element) is filled."""
         n = self.numDMs * self.block_samples + 1
         if dtype == np.complex64:
-            buf = out if out is not None else np.zeros(n, np.complex64)
+            buf = out if out is not None else _pinned.empty(n, np.complex64)
             assert buf.dtype == np.complex64 and buf.size == n and buf.flags.c_contiguous
             check(lib().msosm_dedisp_get_output_c64(self._h, buf.ctypes.data))
             return buf if out is not None else buf[:-1].reshape(self.numDMs, self.block_samples)
-        buf = out if out is not None else np.zeros((n, 2), np.uint16)
+        buf = out if out is not None else _pinned.empty((n, 2), np.uint16)
         assert buf.dtype == np.uint16 and buf.size == 2 * n and buf.flags.c_contiguous
         check(lib().msosm_dedisp_get_output_uint16(self._h, buf.ctypes.data))
         return buf if out is not None else buf[:-1].reshape(self.numDMs, self.block_samples, 2)
@@ -191,7 +191,7 @@ class Dedisperser:
         self.folding = True
 
     def get_profiles(self) -> np.ndarray:
-        out = np.zeros((self.numDMs, self.time_bin), np.float32)
+        out = _pinned.empty((self.numDMs, self.time_bin), np.float32)
         check(lib().msosm_dedisp_get_profiles(self._h, out.ctypes.data))
         return out
 

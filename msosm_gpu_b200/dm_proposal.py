@@ -24,7 +24,7 @@ from typing import Optional, Sequence
 
 import numpy as np
 
-from . import _abi
+from . import _abi, _pinned
 from ._abi import check, lib
 
 OFFSET_CLIP = 3.0  # coarse steps
@@ -68,7 +68,7 @@ class DMProposalNet:
     def gradient(self, x, label, target, want_grad: bool = False):
         B = x.shape[0]
         loss = ctypes.c_float()
-        g = np.empty(self.n_params, np.float32) if want_grad else None
+        g = _pinned.empty(self.n_params, np.float32) if want_grad else None
         check(lib().msosm_cnn_gradient(self._h, _ptr(x), _ptr(label), _ptr(target), B, ctypes.byref(loss),
                                        None if g is None else g.ctypes.data))
         return float(loss.value), g
