@@ -216,6 +216,14 @@ __global__ void __launch_bounds__(PairShape<LOG2N>::THREADS, PairShape<LOG2N>::C
             __syncwarp();
             tmem_st_32(tm + P::COL_H, h);
             tmem_st_16(tm + P::COL_D, d);
+        } else {
+            // the block delays of bins j + r T and M further, one word
+            uint32_t d[16];
+#pragma unroll
+            for (int r = 0; r < 16; ++r)
+                d[r] = (uint32_t)__ldg(dl + r * T) | (uint32_t)__ldg(dl + M + r * T) << 16;
+            __syncwarp();
+            tmem_st_16(tm + P::COL_D, d);
         }
         FoldCursor cursor;
         if constexpr (FOLD) {
@@ -264,6 +272,18 @@ __global__ void __launch_bounds__(PairShape<LOG2N>::THREADS, PairShape<LOG2N>::C
                         if (two && kg + 1 >= d)
                             xb[r] = base[(size_t)((slot - d + 1) & smask) * N + r * T];
                     }
+                }
+            } else if (kg >= a.max_delay && small_ring) {
+                uint32_t d[16];
+                tmem_ld_16(tm + P::COL_D, d);
+                const char *ring = reinterpret_cast<const char *>(a.ring + j);
+#pragma unroll
+                for (int r = 0; r < 16; ++r) {
+                    constexpr uint32_t ROW = (uint32_t)(N * sizeof(float2));
+                    const uint32_t o0 = (uint32_t)((slot - (int)(d[r] & 0xFFFFu)) & smask) * ROW;
+                    const uint32_t o1 = (uint32_t)((slot - (int)(d[r] >> 16)) & smask) * ROW;
+                    xa[r] = reinterpret_cast<const float2 *>(ring + o0)[r * T];
+                    xb[r] = reinterpret_cast<const float2 *>(ring + o1)[M + r * T];
                 }
             } else {
 #pragma unroll
