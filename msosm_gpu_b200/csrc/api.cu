@@ -10,6 +10,7 @@
 #include <new>
 #include <string>
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -72,6 +73,18 @@ bool is_device_ptr(const void *p)
     return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
 }
 
+// The device address of page-locked host memory, null for any other
+template <typename T>
+T *mapped_host(T *p)
+{
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return at.type == cudaMemoryTypeHost ? static_cast<T *>(at.devicePointer) : nullptr;
+}
+
 // exp(sign * 2 pi i e / n), e < n, computed in double on the host
 std::vector<float2> twiddle_table(int n, int sign)
 {
@@ -122,7 +135,7 @@ struct msosm_dedisp {
     float2 *ring = nullptr, *H = nullptr, *hist = nullptr, *series_buf = nullptr;
     uint16_t *delays_d = nullptr;
     float2 *tw_fwd = nullptr, *tw_inv = nullptr, *tw_inv_m = nullptr;
-    int *work = nullptr;  // the dedispersion kernel's item counter (DedispArgs::work)
+    int *work = nullptr;  // the dedispersion kernel's item counter (DedispArgs::work), behind hist
     void *staging[2] = {nullptr, nullptr};
     uint32_t *u16_out = nullptr;
     // folding
@@ -143,6 +156,7 @@ struct msosm_dedisp {
     // a timed-out wait in the kernel
     bool tc = false, tc_bf16 = false;
     int *status_d = nullptr;
+    int *status_h = nullptr;  // page-locked: the status as of the last synchronising call
     long long tc_wait_limit_ns = kTcWaitLimitDefaultNs;  // each wait of the kernel on a GEMM
     float *row_max = nullptr;  // [S] largest |component| of each ring row
     float *h_max = nullptr;    // [D] largest |component| of each trial's H
@@ -166,6 +180,34 @@ struct msosm_dedisp {
 
 namespace {
 
+// Page-locked words for the handles' status: slots of 4 KB pages (a page-locked
+// allocation costs about a millisecond), taken and given back under a lock; a
+// page per 1024 handles alive at one time.
+std::mutex g_slot_lock;
+std::vector<int *> g_slots;
+
+cudaError_t status_slot(int **out)
+{
+    const std::lock_guard<std::mutex> lock(g_slot_lock);
+    if (g_slots.empty()) {
+        int *page = nullptr;
+        const cudaError_t e = cudaHostAlloc((void **)&page, 1024 * sizeof(int), cudaHostAllocPortable);
+        if (e != cudaSuccess)
+            return e;
+        for (int i = 1023; i >= 0; --i)
+            g_slots.push_back(page + i);
+    }
+    *out = g_slots.back();
+    g_slots.pop_back();
+    return cudaSuccess;
+}
+
+void status_slot_free(int *slot)
+{
+    const std::lock_guard<std::mutex> lock(g_slot_lock);
+    g_slots.push_back(slot);
+}
+
 void release(msosm_dedisp *d)
 {
     if (!d)
@@ -177,13 +219,15 @@ void release(msosm_dedisp *d)
     void *bufs[] = {d->ring, d->H, d->hist, d->series_buf, d->delays_d, d->tw_fwd, d->tw_inv, d->tw_inv_m,
                     d->staging[0], d->staging[1], d->u16_out, d->part_main, d->part_pend, d->prof_out,
                     d->acc_main, d->acc_pend, d->span_a_d, d->span_b_d, d->span_p_d, d->span_dest_d,
-                    d->work, d->lA, d->lB, d->lI, d->tw1f, d->tw1i, d->tw2f, d->tw2i, d->status_d,
+                    d->lA, d->lB, d->lI, d->tw1f, d->tw1i, d->tw2f, d->tw2i, d->status_d,
                     d->row_max, d->h_max, d->delay_max_d};
     for (void *p : bufs)
         if (p)
             cudaFree(p);
     if (d->span_host)
         cudaFreeHost(d->span_host);
+    if (d->status_h)
+        status_slot_free(d->status_h);
     for (int i = 0; i < 2; ++i) {
         if (d->ev_copied[i])
             cudaEventDestroy(d->ev_copied[i]);
@@ -709,8 +753,10 @@ msosm_status msosm_dedisp_create(const float *bw, const float *dm, const float *
     CKD(dalloc(&d->ring, (size_t)d->S * N, tot));
     CKD(dalloc(&d->H, (size_t)numDMs * N, tot));
     CKD(dalloc(&d->delays_d, (size_t)numDMs * N, tot));
-    CKD(dalloc(&d->hist, 2 * (size_t)M, tot));
-    CKD(cudaMemsetAsync(d->hist, 0, sizeof(float2) * 2 * M, d->stream));
+    // the history and, behind it, the dedispersion kernel's two counters
+    CKD(dalloc(&d->hist, 2 * (size_t)M + 1, tot));
+    CKD(cudaMemsetAsync(d->hist, 0, sizeof(float2) * (2 * M + 1), d->stream));
+    d->work = reinterpret_cast<int *>(d->hist + 2 * M);
     for (int i = 0; i < 2; ++i)
         CKD(dalloc((float2 **)&d->staging[i], (size_t)count * M, tot));
     if (d->series) {
@@ -749,8 +795,6 @@ msosm_status msosm_dedisp_create(const float *bw, const float *dm, const float *
             release(d);
             return s;
         }
-        CKD(dalloc(&d->work, 2, tot));
-        CKD(cudaMemsetAsync(d->work, 0, 2 * sizeof(int), d->stream));
         if ((s = design_filters(log2n, cp, scale, sign, d->tw_inv_m, d->tw_fwd, d->H, d->stream)) != MSOSM_OK) {
             release(d);
             return s;
@@ -768,6 +812,7 @@ msosm_status msosm_dedisp_create(const float *bw, const float *dm, const float *
             CKD(e);
             CKD(dalloc(&d->status_d, 1, tot));
             CKD(cudaMemset(d->status_d, 0, sizeof(int)));
+            CKD(status_slot(&d->status_h));
             // scale bounds: ring rows not yet written hold zero
             CKD(dalloc(&d->row_max, (size_t)d->S, tot));
             CKD(cudaMemset(d->row_max, 0, sizeof(float) * d->S));
@@ -1036,17 +1081,16 @@ static msosm_status filter_block_large(msosm_dedisp *d, const void *src, InputKi
     return MSOSM_OK;
 }
 
-// After the handle's stream has drained: a timed-out wait of the
-// tensor-core kernel (the results of the calls since the last check are then
-// invalid).  The status word is cleared once reported, so the handle goes
-// on with the next call.
-static msosm_status kernel_status(msosm_dedisp *d)
+// Drains the handle's stream and reports a timed-out wait of the tensor-core
+// kernel (the results of the calls since the last check are then invalid).
+// The status word comes back behind whatever copy the caller has queued; it
+// is cleared once reported, so the handle goes on with the next call.
+static msosm_status drain(msosm_dedisp *d)
 {
-    if (!d->status_d)
-        return MSOSM_OK;
-    int st = 0;
-    CK(cudaMemcpy(&st, d->status_d, sizeof(int), cudaMemcpyDeviceToHost));
-    if (st != 0) {
+    if (d->status_d)
+        CK(cudaMemcpyAsync(d->status_h, d->status_d, sizeof(int), cudaMemcpyDeviceToHost, d->stream));
+    CK(cudaStreamSynchronize(d->stream));
+    if (d->status_d && *d->status_h != 0) {
         CK(cudaMemset(d->status_d, 0, sizeof(int)));
         return fail(MSOSM_ERR_TIMEOUT, "tensor-core kernel: a wait on the tensor core timed out");
     }
@@ -1411,7 +1455,7 @@ msosm_status msosm_batch_synchronize(msosm_batch *b)
         return fail(MSOSM_ERR_BAD_ARG, "null batch");
     CK(cudaStreamSynchronize(b->stream));
     for (msosm_dedisp *d : b->h) {
-        msosm_status st = kernel_status(d);
+        msosm_status st = drain(d);
         if (st != MSOSM_OK)
             return st;
     }
@@ -1436,8 +1480,7 @@ msosm_status msosm_dedisp_get_output_c64(msosm_dedisp *d, msosm_complex *out)
         return fail(MSOSM_ERR_STATE, "handle created with MSOSM_FLAG_NO_SERIES");
     const size_t n = (size_t)d->D * d->count * d->M + 1;
     CK(cudaMemcpyAsync(out, d->series_buf, sizeof(float2) * n, cudaMemcpyDeviceToHost, d->stream));
-    CK(cudaStreamSynchronize(d->stream));
-    return kernel_status(d);
+    return drain(d);
 }
 
 msosm_status msosm_dedisp_get_output_uint16(msosm_dedisp *d, msosm_uint16_pair *out)
@@ -1451,8 +1494,7 @@ msosm_status msosm_dedisp_get_output_uint16(msosm_dedisp *d, msosm_uint16_pair *
         CK(dalloc(&d->u16_out, n, d->device_bytes));
     CK(launch_encode_u16(d->series_buf, d->u16_out, n, d->stream));
     CK(cudaMemcpyAsync(out, d->u16_out, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, d->stream));
-    CK(cudaStreamSynchronize(d->stream));
-    return kernel_status(d);
+    return drain(d);
 }
 
 msosm_status msosm_dedisp_output_device_ptr(msosm_dedisp *d, msosm_complex **ptr)
@@ -1586,10 +1628,12 @@ msosm_status msosm_dedisp_get_profiles(msosm_dedisp *d, float *out)
     if (!d->fold)
         return fail(MSOSM_ERR_STATE, "fold not configured (msosm_dedisp_fold_init)");
     const size_t n = (size_t)d->D * d->nbins;
-    CK(launch_fold_readout(d->acc_main, n, d->out_scale, d->prof_out, d->stream));
-    CK(cudaMemcpyAsync(out, d->prof_out, sizeof(float) * n, cudaMemcpyDeviceToHost, d->stream));
-    CK(cudaStreamSynchronize(d->stream));
-    return kernel_status(d);
+    // page-locked memory is written by the kernel itself
+    float *direct = mapped_host(out);
+    CK(launch_fold_readout(d->acc_main, n, d->out_scale, direct ? direct : d->prof_out, d->stream));
+    if (!direct)
+        CK(cudaMemcpyAsync(out, d->prof_out, sizeof(float) * n, cudaMemcpyDeviceToHost, d->stream));
+    return drain(d);
 }
 
 msosm_status msosm_dedisp_folded_periods(const msosm_dedisp *d, unsigned long long *n)
@@ -1604,9 +1648,8 @@ msosm_status msosm_dedisp_synchronize(msosm_dedisp *d)
 {
     if (check_handle(d))
         return MSOSM_ERR_BAD_ARG;
-    CK(cudaStreamSynchronize(d->stream));
     CK(cudaStreamSynchronize(d->copy_stream));
-    return kernel_status(d);
+    return drain(d);
 }
 
 msosm_status msosm_dedisp_enable_timing(msosm_dedisp *d, int on)
