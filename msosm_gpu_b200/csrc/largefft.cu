@@ -48,10 +48,12 @@ __device__ __forceinline__ float2 twiddle_n(int e, int log2n, float sign)
 }
 
 // v[slot] *= W_N^(sign a k), k = j + m T the output index of the slot
-// (last_out_index: slot q R + r holds m = q + r 16/R).  Five sines and cosines and at most
-// three products per factor instead of sixteen: those, with the 64-bit
+// (last_out_index: slot q R + r holds m = q + r 16/R).  Seven sines and cosines and one
+// product per factor instead of sixteen sines and cosines: those, with the 64-bit
 // indices, were most of the column pass's instructions (54 us for 32 windows
-// of 2^18 points).
+// of 2^18 points).  One call at 2^18: 144.6 us, with sixteen 159.3, with five and up to
+// three products 143.3, but there the profile's error against FP64 grew from 6.0e-7
+// to 6.1e-7; with one product it is 6.0e-7 as with sixteen.
 template <int LOG2L>
 __device__ __forceinline__ void twiddle_outputs(float2 (&v)[16], int a, int j, int log2n, float sign)
 {
@@ -59,13 +61,12 @@ __device__ __forceinline__ void twiddle_outputs(float2 (&v)[16], int a, int j, i
     constexpr int R = F::radix(F::NST - 1), B = 16 / R;
     const int s = a * F::T;
     float2 b[4];
-    b[1] = twiddle_n(s, log2n, sign);
-    b[2] = cmul(b[1], b[1]);
-    b[3] = cmul(b[2], b[1]);
-    const float2 w0 = twiddle_n(a * j, log2n, sign);
+#pragma unroll
+    for (int m1 = 1; m1 < 4; ++m1)
+        b[m1] = twiddle_n(m1 * s, log2n, sign);
 #pragma unroll
     for (int m4 = 0; m4 < 4; ++m4) {
-        const float2 c = m4 == 0 ? w0 : cmul(w0, twiddle_n(4 * m4 * s, log2n, sign));
+        const float2 c = twiddle_n(a * (j + 4 * m4 * F::T), log2n, sign);
 #pragma unroll
         for (int m1 = 0; m1 < 4; ++m1) {
             const int m = 4 * m4 + m1, slot = (m % B) * R + m / B;
