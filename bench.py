@@ -419,7 +419,7 @@ def run_ours(args):
         ach = flops_per_sample * launch_samples / (k_ms * 1e-3) / 1e12
         return {"bound": "fp32", "achieved": ach, "peak": fp32, "unit": "TFLOP/s",
                 "frac": ach / fp32 if fp32 else None,
-                "kernel": f"dedisp_kernel<{log2n}> (gather x H, FP32 shared-memory inverse FFT, discard, |y|^2, fold)",
+                "kernel": f"pair_dedisp_kernel<{log2n}> (gather x H, packed FP32 inverse FFT, discard, |y|^2, fold)",
                 "flops_per_dm_sample": flops_per_sample, "kernel_ms": k_ms,
                 "peak_source": "cuBLAS SGEMM 8192^3 measured in this run (MEASURED_PEAKS.json has no FP32 figure)",
                 "stage_ms_per_step": stages(t)}
