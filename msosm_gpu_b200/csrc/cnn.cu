@@ -205,7 +205,8 @@ __global__ void __launch_bounds__(64) conv_kernel(const float *__restrict__ in, 
 // output x 8 input channels: each lane holds 4 output x 2 input channels x K
 // taps in registers (co = lane % 8 + 8 i, ci = 2 (lane / 8) + {0, 1}, the two
 // input channels as a packed pair), the four warps a quarter of the phases
-// each, so that 9 16-byte reads of shared memory feed 16 K packed FMAs.  Warps are added in order, groups by wgrad_reduce_kernel in order.
+// each, so that 9 16-byte reads of shared memory feed 16 K packed FMAs.  Warps are added in order, groups by wgrad_reduce_kernel in
+// order.
 // Bound by the FP32 lanes and shared memory.  256 samples x 256 phases, 64 ->
 // 32 channels, 7 taps: 60 us, 820 before (one block per (co, ci), every
 // product's operands read from memory).
@@ -365,14 +366,30 @@ __global__ void __launch_bounds__(128, K <= 7 ? 4 : 2) conv_wgrad_kernel(const f
     }
 }
 
-// Sum of the groups' rows; n values (weights then biases, as they lie in the
-// gradient).  Eight slices of the rows per value, added in order.
-__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float *__restrict__ part, int groups, long long n,
-                                                           float *__restrict__ out)
+// Partial rows of the layers' weight gradients: row r of layer l at part +
+// offset[l] + r n, n = values[l] weights then biases, as they lie in the
+// gradient at out[l].
+constexpr int kMaxLayers = 16;
+
+struct WgradRows {
+    const float *part;
+    float *grad;
+    long long offset[kMaxLayers], out[kMaxLayers], values[kMaxLayers];
+    int groups[kMaxLayers];
+};
+
+// Sum of the groups' rows of every layer (blockIdx.y) in one launch after the
+// backward pass.  Eight slices of the rows per value, added in order.  Bound by
+// latency: a launch per layer, each between two convolutions, took 5 - 7 us (a
+// gradient of 256 samples and four layers 459 us, with one launch 442).
+__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const __grid_constant__ WgradRows rows)
 {
     __shared__ float sums[8][32];
-    const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
-    const long long i = (long long)blockIdx.x * 32 + lane;
+    const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5, l = blockIdx.y, groups = rows.groups[l];
+    const long long i = (long long)blockIdx.x * 32 + lane, n = rows.values[l];
+    if ((long long)blockIdx.x * 32 >= n)
+        return;
+    const float *__restrict__ part = rows.part + rows.offset[l];
     float s = 0.f;
     if (i < n) {
 #pragma unroll 4
@@ -385,7 +402,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float *__restri
 #pragma unroll
         for (int k = 1; k < 8; ++k)
             s += sums[k][lane];
-        out[i] = s;
+        rows.grad[rows.out[l] + i] = s;
     }
 }
 
@@ -434,8 +451,8 @@ cudaError_t launch_conv(int K, const float *in, int Cin, int L, const float *w, 
     });
 }
 
-// dw (then db) of one layer into grad, through the partial rows
-cudaError_t launch_wgrad(int K, const float *g, int Co, const float *a, int Ci, int B, int L, float *part, float *grad,
+// dw (then db) of one layer into its partial rows
+cudaError_t launch_wgrad(int K, const float *g, int Co, const float *a, int Ci, int B, int L, float *part,
                          cudaStream_t st)
 {
     return with_taps(K, [&](auto taps) -> cudaError_t {
@@ -447,11 +464,6 @@ cudaError_t launch_wgrad(int K, const float *g, int Co, const float *a, int Ci, 
         if (e != cudaSuccess)
             return e;
         k<<<dim3(Ci / kWgCi, (Co + kWgCo - 1) / kWgCo, groups), 128, sm, st>>>(g, Co, a, Ci, B, L, groups, part);
-        e = cudaGetLastError();
-        if (e != cudaSuccess)
-            return e;
-        const long long n = (long long)Co * Ci * KK + Co;
-        wgrad_reduce_kernel<<<(unsigned)((n + 31) / 32), 256, 0, st>>>(part, groups, n, grad);
         return cudaGetLastError();
     });
 }
@@ -689,7 +701,8 @@ struct msosm_cnn {
     __nv_bfloat16 *q = nullptr;
     std::vector<float *> act;        // act[1..layers]: [max_batch][C][L]
     float *xin = nullptr, *lab = nullptr, *tgt = nullptr;  // staged host inputs
-    float *part = nullptr;           // partial rows of one layer's weight gradient
+    float *part = nullptr;           // partial rows of the weight gradients, layer l's from part_off[l]
+    std::vector<long long> part_off;
     float *g0 = nullptr, *g1 = nullptr;  // gradient ping-pong [max_batch][max(Cin, C)][L]
     float *wf = nullptr, *wb = nullptr;  // packed weights (PackArgs)
     float *h = nullptr, *dl = nullptr, *dof = nullptr, *logit = nullptr, *off = nullptr, *loss = nullptr;
@@ -762,7 +775,7 @@ msosm_status msosm_cnn_create(const msosm_cnn_config *cfg, unsigned long long se
     if (g.in_channels < 1 || g.in_channels > 256 || g.length < 32 || g.length > 1024 || g.length % 32 != 0 ||
         g.channels < kCoBlock || g.channels > 256 || g.channels % kCoBlock != 0 || g.in_channels % kCoBlock != 0 ||
         g.kernel < 1 || g.kernel > 15 || g.kernel % 2 == 0 || g.kernel > g.length || g.layers < 1 ||
-        g.layers > 16 || g.max_batch < 1 || g.max_batch > 1024 || !(g.dm_weight >= 0.f))
+        g.layers > kMaxLayers || g.max_batch < 1 || g.max_batch > 1024 || !(g.dm_weight >= 0.f))
         return cfail(MSOSM_ERR_BAD_ARG,
                      "cnn: in_channels and channels multiples of 8 (<= 256), length a multiple of 32 in 32 .. 1024, "
                      "odd kernel <= 15, 1 .. 16 layers, max_batch 1 .. 1024, dm_weight >= 0");
@@ -846,12 +859,13 @@ msosm_status msosm_cnn_create(const msosm_cnn_config *cfg, unsigned long long se
     al(&c->logit, B);
     al(&c->off, B);
     al(&c->loss, 1);
-    // partial rows of the widest layer's weight gradient
+    // partial rows of the weight gradients
     size_t prows = 0;
     for (int l = 0; l < g.layers; ++l) {
         const int cin = l == 0 ? g.in_channels : g.channels;
         const size_t n = (size_t)g.channels * cin * g.kernel + g.channels;
-        prows = std::max(prows, n * (size_t)wgrad_groups(g.channels, cin, g.max_batch));
+        c->part_off.push_back((long long)prows);
+        prows += n * (size_t)wgrad_groups(g.channels, cin, g.max_batch);
     }
     al(&c->part, prows);
     if (e == cudaSuccess)
@@ -989,17 +1003,30 @@ msosm_status msosm_cnn_gradient(msosm_cnn *c, const float *x, const float *label
             (unsigned)C, (unsigned)L / 4, (unsigned)n4, (float)L, reinterpret_cast<float4 *>(gcur));
         e = cudaGetLastError();
     }
+    WgradRows rows{};
+    rows.part = c->part;
+    rows.grad = c->grad;
+    long long widest = 0;
     for (int l = g.layers - 1; l >= 0 && e == cudaSuccess; --l) {
         const int ci = l == 0 ? g.in_channels : C;
         const float *a_in = l == 0 ? xd : c->act[l];
         // weights and biases of a layer lie together in the gradient
-        e = launch_wgrad(K, gcur, C, a_in, ci, batch, L, c->part, c->grad + c->w_off[l], c->st);
+        rows.offset[l] = c->part_off[l];
+        rows.out[l] = c->w_off[l];
+        rows.values[l] = (long long)C * ci * K + C;
+        rows.groups[l] = wgrad_groups(C, ci, batch);
+        widest = std::max(widest, rows.values[l]);
+        e = launch_wgrad(K, gcur, C, a_in, ci, batch, L, c->part + c->part_off[l], c->st);
         if (e == cudaSuccess && l > 0) {
             e = launch_conv<true>(K, gcur, C, L, c->wb + c->w_off[l], nullptr, ci, batch, c->act[l], gnext, c->st);
             float *t = gcur;
             gcur = gnext;
             gnext = t;
         }
+    }
+    if (e == cudaSuccess) {
+        wgrad_reduce_kernel<<<dim3((unsigned)((widest + 31) / 32), (unsigned)g.layers), 256, 0, c->st>>>(rows);
+        e = cudaGetLastError();
     }
     if (e == cudaSuccess && loss)
         e = cudaMemcpyAsync(loss, c->loss, sizeof(float), cudaMemcpyDefault, c->st);

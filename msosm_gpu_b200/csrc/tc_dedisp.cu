@@ -1,7 +1,7 @@
 // tc_dedisp.cu -- tensor-core (tcgen05) variant of the fused dedispersion
 // kernel for 4096-, 8192- and 16384-point transforms.
 //
-// Same semantics as dedisp_kernel (kernels.cu), which replaces
+// Same semantics as pair_dedisp_kernel (pair_dedisp.cu), which replaces
 // ComplexMultiplyDelay_concurrent_batch + inverse cufftExecC2C +
 // DiscardSamples_concurrent_batch (gpu/gpu_kernel.cu:128-198,236-258) and the
 // host fold of Fold_GPU (folding/fold_gpu.cpp:48-194): per (trial, block)
