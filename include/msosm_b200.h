@@ -284,8 +284,9 @@ MSOSM_API msosm_status msosm_fold_discard_samples(msosm_fold *f, unsigned long N
  * be NULL for one polarisation) into the fold's buffer.  Replaces
  * Fold_GPU::calculate_intensity (fold_gpu.cpp:35-43) and calculateIntensity
  * (gpu/gpu_kernel.cu:347-353); the result stays on the device.  The raw
- * pointers carry no ordering, so this waits for the whole device first; with
- * dedisperser handles use msosm_fold_calculate_intensity_dedisp. */
+ * pointers carry no ordering, so this waits for the whole device first and
+ * for its own read at the end (a and b may be overwritten or freed once it
+ * returns); with dedisperser handles use msosm_fold_calculate_intensity_dedisp. */
 MSOSM_API msosm_status msosm_fold_calculate_intensity(msosm_fold *f, const msosm_complex *a, const msosm_complex *b);
 /* Same from the last series of one or two dedisperser handles (each
  * count*M == size samples, one trial; b may be NULL), ordered after their

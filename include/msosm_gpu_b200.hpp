@@ -606,13 +606,18 @@ public:
     // MSOSM_GPU_BATCH / OSM_GPU_BATCH: ordered after their last filter call
     void calculate_intensity(MSOSM_GPU_BATCH *pol1, MSOSM_GPU_BATCH *pol2)
     {
-        check(msosm_fold_calculate_intensity_dedisp(h_, pol1->handle(), pol2 ? pol2->handle() : nullptr),
-              "calculate_intensity");
+        by_handle(pol1, pol2);
     }
-    // any other class with a device output_buffer_d (waits for the device)
+    // OSM_GPU_BATCH, calculate_intensity<MSOSM_GPU_BATCH>(..): the same, when
+    // their series are as long as the fold's chunk; any other class with a
+    // device output_buffer_d: the first size samples (waits for the device)
     template <typename T>
     void calculate_intensity(T *pol1, T *pol2)
     {
+        if (whole_series(pol1) && (!pol2 || whole_series(pol2))) {
+            by_handle(pol1, pol2);
+            return;
+        }
         check(msosm_fold_calculate_intensity(h_, pol1->output_buffer_d, pol2 ? pol2->output_buffer_d : nullptr),
               "calculate_intensity");
     }
@@ -651,6 +656,16 @@ public:
     bool track_raw_state = false;
 
 private:
+    void by_handle(MSOSM_GPU_BATCH *pol1, MSOSM_GPU_BATCH *pol2)
+    {
+        check(msosm_fold_calculate_intensity_dedisp(h_, pol1->handle(), pol2 ? pol2->handle() : nullptr),
+              "calculate_intensity");
+    }
+    void by_handle(void *, void *) {}
+    // whether p is a single-DM object whose series is one chunk
+    bool whole_series(const MSOSM_GPU_BATCH *p) const { return (unsigned long)p->count * p->M == size_; }
+    bool whole_series(const void *) const { return false; }
+
     // the chunk's destinations from the same fold state machine the device
     // fold follows (msosm_fold_planner_chunk), applied to its intensities
     void track_chunk()

@@ -1827,6 +1827,8 @@ msosm_status msosm_fold_calculate_intensity(msosm_fold *f, const msosm_complex *
     CK(cudaDeviceSynchronize());
     CK(launch_intensity(reinterpret_cast<const float2 *>(a), reinterpret_cast<const float2 *>(b), f->I, f->size,
                         f->stream));
+    // nor is it known who writes or frees them next: done reading on return
+    CK(cudaStreamSynchronize(f->stream));
     return MSOSM_OK;
 }
 
