@@ -63,19 +63,27 @@ __device__ __forceinline__ void cp_async4(float *dst, const float *src)
 constexpr int kT = 8;
 constexpr int kCiChunk = 16;
 
-// A block: tt threads across the phases, cg across the channels.
-struct ConvShape {
-    int tt, cg;
-    ConvShape(int channels, int L)
-    {
-        tt = L > 64 ? 16 : (L > 32 ? 8 : 4);
-        cg = channels / kCoBlock < 64 / tt ? channels / kCoBlock : 64 / tt;
-    }
-};
 // a block's input row in shared memory: phase tb + i at kXLead + i, so that
 // its 16-byte vectors lie as in memory; the taps reach K/2 to either side
 constexpr int kXLead = 8;
 __host__ __device__ constexpr int conv_xw(int tt) { return kT * tt + 2 * kXLead + 4; }
+
+// A block: tt threads across the phases, cg across the channels; 64 threads,
+// or fewer for few channels or where the weights of that many channels do not
+// fit (32 phases, 15 taps, 120 channels and more: half of the channel groups).
+struct ConvShape {
+    int tt, cg;
+    ConvShape(int channels, int L, int K)
+    {
+        tt = L > 64 ? 16 : (L > 32 ? 8 : 4);
+        cg = channels / kCoBlock < 64 / tt ? channels / kCoBlock : 64 / tt;
+        while (cg > 1 && smem(K) > kConvSmemMax)
+            cg = (cg + 1) / 2;
+    }
+    // both stages: kCiChunk input rows and their weights
+    size_t smem(int K) const { return sizeof(float) * 2 * kCiChunk * ((size_t)conv_xw(tt) + (size_t)K * kCoBlock * cg); }
+    static constexpr size_t kConvSmemMax = 227 * 1024;  // a block's share of sm_100a
+};
 
 using pairfft::f2;
 
@@ -437,9 +445,9 @@ cudaError_t launch_conv(int K, const float *in, int Cin, int L, const float *w, 
 {
     return with_taps(K, [&](auto taps) -> cudaError_t {
         constexpr int KK = decltype(taps)::value;
-        const ConvShape shape(Cout, L);
+        const ConvShape shape(Cout, L, KK);
         const int cg = shape.cg, tt = shape.tt;
-        const size_t sm = sizeof(float) * 2 * kCiChunk * ((size_t)conv_xw(tt) + (size_t)KK * kCoBlock * cg);
+        const size_t sm = shape.smem(KK);
         auto k = conv_kernel<KK, BWD>;
         cudaError_t e = allow_smem(k, sm);
         if (e != cudaSuccess)
