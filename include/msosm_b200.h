@@ -186,7 +186,10 @@ MSOSM_API msosm_status msosm_dedisp_set_stream(msosm_dedisp *d, void *stream);
 /* Dedisperse the next count*M samples (all trials).  Replaces
  * filter_block_uint16 (msosm_gpu_dm_concurrent.cpp:119-151,
  * msosm_gpu_batch.cpp:75-94, osm_gpu_batch.cpp:94-123).  The input is
- * offset-binary (x == 0 is blank, else x - 32768). */
+ * offset-binary (x == 0 is blank, else x - 32768).  A handle created with
+ * MSOSM_FLAG_NO_SERIES needs msosm_dedisp_fold_init first (MSOSM_ERR_STATE
+ * otherwise at FFT sizes up to 16384; above, the samples only enter the
+ * stream's history). */
 MSOSM_API msosm_status msosm_dedisp_filter_block_uint16(msosm_dedisp *d, const msosm_uint16_pair *input);
 /* Same for complex64 input (the reference has no such entry point). */
 MSOSM_API msosm_status msosm_dedisp_filter_block_c64(msosm_dedisp *d, const msosm_complex *input);

@@ -1193,10 +1193,21 @@ static msosm_status call_end(msosm_dedisp *d, msosm_dedisp::CallEvents *ev, int 
     return MSOSM_OK;
 }
 
+// A handle without series whose fold is not configured has nowhere to write:
+// the block FFT kernels are built for at least one of the two outputs.
+static msosm_status check_outputs(const msosm_dedisp *d)
+{
+    if (!d->series && !d->fold && !d->large)
+        return fail(MSOSM_ERR_STATE, "handle created with MSOSM_FLAG_NO_SERIES: call msosm_dedisp_fold_init first");
+    return MSOSM_OK;
+}
+
 static msosm_status filter_block(msosm_dedisp *d, const void *input, InputKind kind)
 {
     if (check_handle(d) || !input)
         return fail(MSOSM_ERR_BAD_ARG, "null handle or input");
+    if (check_outputs(d) != MSOSM_OK)
+        return MSOSM_ERR_STATE;
     msosm_dedisp::CallEvents *ev = nullptr;
     if (d->timing) {
         msosm_dedisp::CallEvents c{};
@@ -1406,6 +1417,9 @@ msosm_status msosm_batch_filter(msosm_batch *b, const void *const *inputs, int i
     for (size_t i = 0; i < b->h.size(); ++i)
         if (!inputs[i])
             return fail(MSOSM_ERR_BAD_ARG, "input %zu is null", i);
+    for (const msosm_dedisp *d : b->h)
+        if (check_outputs(d) != MSOSM_OK)
+            return MSOSM_ERR_STATE;
     // handles outside every group: their whole call, one after another
     for (int i : b->alone) {
         msosm_status st = filter_block(b->h[i], inputs[i], kind);

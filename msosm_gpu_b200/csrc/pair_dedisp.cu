@@ -453,6 +453,8 @@ cudaError_t launch_t(bool series, bool fold, const DedispArgs &a, int grid, cuda
 
 cudaError_t launch_dedisp(int log2n, bool series, bool fold, const DedispArgs &a, int grid, cudaStream_t st)
 {
+    if (!series && !fold)
+        return cudaErrorInvalidValue;
 #define CALL(L) launch_t<L>(series, fold, a, grid, st)
     MSOSM_PAIR_DISPATCH(log2n, CALL)
 #undef CALL

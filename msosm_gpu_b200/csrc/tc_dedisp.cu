@@ -1147,7 +1147,7 @@ int tc_blocks_per_sm(int log2n, bool bf16, bool series, bool fold, size_t extra_
 cudaError_t launch_tc_dedisp(int log2n, bool bf16, bool series, bool fold, const DedispArgs &a, int grid,
                              cudaStream_t st)
 {
-    if (!a.status || !tc_supported(log2n))
+    if (!a.status || !tc_supported(log2n) || (!series && !fold))
         return cudaErrorInvalidValue;
     const NoBatch none{};
     const size_t fs = fold ? fold_smem_bytes(a.fold.nbins, a.fold.span_cap, a.fold.smem_prof != 0)
@@ -1162,7 +1162,7 @@ cudaError_t launch_tc_dedisp(int log2n, bool bf16, bool series, bool fold, const
 cudaError_t launch_tc_dedisp_batch(int log2n, bool bf16, bool series, bool fold, const BatchArgs &b,
                                    size_t fold_smem, int grid, cudaStream_t st)
 {
-    if (!b.counter || b.nobs < 1 || b.nobs > kBatchMax || !tc_supported(log2n))
+    if (!b.counter || b.nobs < 1 || b.nobs > kBatchMax || !tc_supported(log2n) || (!series && !fold))
         return cudaErrorInvalidValue;
     DedispArgs none{};
     if (log2n == 14)
