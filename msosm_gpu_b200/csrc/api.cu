@@ -305,6 +305,12 @@ bool prof_in_smem(const msosm_dedisp *d)
     return dedisp_smem(d->log2n, true, fs) <= dedisp_smem_share(d->log2n);
 }
 
+// Shared memory of a work item's fold state, 0 without folding.
+size_t fold_smem(const msosm_dedisp *d)
+{
+    return d->fold ? fold_smem_bytes(d->nbins, d->win_cap, prof_in_smem(d)) : 0;
+}
+
 // Block ranges per trial and the persistent grid of the dedispersion kernel.
 // A work item is one (block range, trial); the grid strides over the items.
 // The ranges are chosen so that the items fill whole waves of the resident
@@ -320,7 +326,7 @@ cudaError_t plan_grid(msosm_dedisp *d)
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess)
         return e;
-    const size_t extra = d->fold ? fold_smem_bytes(d->nbins, d->win_cap, prof_in_smem(d)) : 0;
+    const size_t extra = fold_smem(d);
     int per_sm;
     if (d->tc) {
         per_sm = tc_blocks_per_sm(d->log2n, d->tc_bf16, d->series, d->fold, extra);
@@ -1259,6 +1265,7 @@ struct msosm_batch {
     cudaStream_t stream = nullptr;      // the stream everything runs on
     cudaStream_t own_stream = nullptr;  // the batch's own (the default)
     unsigned long long calls = 0;
+    bool planned = false;  // groups hold the handles as batch_plan saw them
 };
 
 static void batch_release(msosm_batch *b)
@@ -1276,6 +1283,100 @@ static void batch_release(msosm_batch *b)
     if (b->own_stream)
         cudaStreamDestroy(b->own_stream);
     delete b;
+}
+
+// Groups the batch's handles by kernel and cuts their work items, from the
+// handles' present state.
+static msosm_status batch_plan(msosm_batch *b)
+{
+    for (auto &g : b->groups)
+        cudaFree(g.counter_d);
+    b->groups.clear();
+    b->alone.clear();
+    b->planned = false;
+    int dev = 0, sms = 1;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    for (int i = 0; i < (int)b->h.size(); ++i) {
+        const msosm_dedisp *d = b->h[i];
+        if (!d->tc || d->large) {
+            b->alone.push_back(i);
+            continue;
+        }
+        int gi = -1;
+        for (size_t k = 0; k < b->groups.size(); ++k) {
+            const auto &g = b->groups[k];
+            if (g.log2n == d->log2n && g.bf16 == d->tc_bf16 && g.series == d->series && g.fold == d->fold &&
+                (int)g.members.size() < kBatchMax)
+                gi = (int)k;
+        }
+        if (gi < 0) {
+            b->groups.emplace_back();
+            gi = (int)b->groups.size() - 1;
+            auto &g = b->groups.back();
+            g.log2n = d->log2n;
+            g.bf16 = d->tc_bf16;
+            g.series = d->series;
+            g.fold = d->fold;
+        }
+        b->groups[gi].members.push_back(i);
+    }
+    for (auto &g : b->groups) {
+        // each member keeps its own cut of trials into block ranges and its
+        // item order (range-major, so the CTAs working at one time read the
+        // same ring rows, which stay in L2 for every trial), as in its own
+        // calls; members are ordered largest first, so the last items of the
+        // launch are small ones
+        for (int i : g.members)
+            g.fold_smem = std::max(g.fold_smem, fold_smem(b->h[i]));
+        int per_sm = tc_blocks_per_sm(g.log2n, g.bf16, g.series, g.fold, g.fold_smem);
+        if (per_sm < 1)
+            per_sm = 1;
+        const long long resident = (long long)per_sm * sms;
+        std::vector<std::pair<long long, int>> order;
+        for (int i : g.members) {
+            const msosm_dedisp *d = b->h[i];
+            const int bps = tc_blocks_per_step(d->log2n);
+            order.push_back({(long long)d->D * ((d->count + bps - 1) / bps), i});
+        }
+        std::stable_sort(order.begin(), order.end(), [](const auto &x, const auto &y) { return x.first > y.first; });
+        g.members.clear();
+        std::vector<int> prefix(1, 0);
+        for (const auto &o : order) {
+            const msosm_dedisp *d = b->h[o.second];
+            g.members.push_back(o.second);
+            g.R.push_back(d->R);
+            prefix.push_back(prefix.back() + d->D * d->R);
+        }
+        g.items = prefix.back();
+        g.grid = (int)std::min<long long>(g.items, resident);
+        const size_t nm = g.members.size();
+        CK(cudaMalloc((void **)&g.counter_d, sizeof(int)));
+        g.args.reset(new (std::nothrow) BatchArgs{});
+        if (!g.args)
+            return fail(MSOSM_ERR_OOM, "host allocation");
+        g.args->nobs = (int)nm;
+        g.args->counter = g.counter_d;
+        for (size_t j = 0; j <= nm; ++j)
+            g.args->prefix[j] = prefix[j];
+    }
+    b->planned = true;
+    return MSOSM_OK;
+}
+
+// Whether a member was reset or folds otherwise since the plan was made: its
+// group, its block ranges or its shared memory no longer fit.
+static bool batch_stale(const msosm_batch *b)
+{
+    if (!b->planned)
+        return true;
+    for (const auto &g : b->groups)
+        for (size_t j = 0; j < g.members.size(); ++j) {
+            const msosm_dedisp *d = b->h[g.members[j]];
+            if (d->fold != g.fold || d->R != g.R[j] || fold_smem(d) > g.fold_smem)
+                return true;
+        }
+    return false;
 }
 
 msosm_status msosm_batch_create(msosm_dedisp *const *handles, int n, msosm_batch **out)
@@ -1305,81 +1406,17 @@ msosm_status msosm_batch_create(msosm_dedisp *const *handles, int n, msosm_batch
     } while (0)
     CKB(cudaStreamCreateWithFlags(&b->own_stream, cudaStreamNonBlocking));
     b->stream = b->own_stream;
-    int dev = 0, sms = 1;
-    CKB(cudaGetDevice(&dev));
-    CKB(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    for (int i = 0; i < n; ++i) {
-        msosm_dedisp *d = b->h[i];
+    for (msosm_dedisp *d : b->h) {
         // every handle's earlier work is done before the batch's stream takes over
         CKB(cudaStreamSynchronize(d->stream));
         d->stream = b->stream;
-        if (!d->tc || d->large) {
-            b->alone.push_back(i);
-            continue;
-        }
-        int gi = -1;
-        for (size_t k = 0; k < b->groups.size(); ++k) {
-            const auto &g = b->groups[k];
-            if (g.log2n == d->log2n && g.bf16 == d->tc_bf16 && g.series == d->series && g.fold == d->fold &&
-                (int)g.members.size() < kBatchMax)
-                gi = (int)k;
-        }
-        if (gi < 0) {
-            b->groups.emplace_back();
-            gi = (int)b->groups.size() - 1;
-            auto &g = b->groups.back();
-            g.log2n = d->log2n;
-            g.bf16 = d->tc_bf16;
-            g.series = d->series;
-            g.fold = d->fold;
-        }
-        b->groups[gi].members.push_back(i);
-    }
-    for (auto &g : b->groups) {
-        // each member keeps its own cut of trials into block ranges and its
-        // item order (range-major, so the CTAs working at one time read the
-        // same ring rows, which stay in L2 for every trial), as in its own
-        // calls; members are ordered largest first, so the last items of the
-        // launch are small ones
-        for (int i : g.members) {
-            const msosm_dedisp *d = b->h[i];
-            if (g.fold)
-                g.fold_smem = std::max(g.fold_smem, fold_smem_bytes(d->nbins, d->win_cap, prof_in_smem(d)));
-        }
-        int per_sm = tc_blocks_per_sm(g.log2n, g.bf16, g.series, g.fold, g.fold_smem);
-        if (per_sm < 1)
-            per_sm = 1;
-        const long long resident = (long long)per_sm * sms;
-        std::vector<std::pair<long long, int>> order;
-        for (int i : g.members) {
-            const msosm_dedisp *d = b->h[i];
-            const int bps = tc_blocks_per_step(d->log2n);
-            order.push_back({(long long)d->D * ((d->count + bps - 1) / bps), i});
-        }
-        std::stable_sort(order.begin(), order.end(), [](const auto &x, const auto &y) { return x.first > y.first; });
-        g.members.clear();
-        std::vector<int> prefix(1, 0);
-        for (const auto &o : order) {
-            const msosm_dedisp *d = b->h[o.second];
-            g.members.push_back(o.second);
-            g.R.push_back(d->R);
-            prefix.push_back(prefix.back() + d->D * d->R);
-        }
-        g.items = prefix.back();
-        g.grid = (int)std::min<long long>(g.items, resident);
-        const size_t nm = g.members.size();
-        CKB(cudaMalloc((void **)&g.counter_d, sizeof(int)));
-        g.args.reset(new (std::nothrow) BatchArgs{});
-        if (!g.args) {
-            batch_release(b);
-            return fail(MSOSM_ERR_OOM, "host allocation");
-        }
-        g.args->nobs = (int)nm;
-        g.args->counter = g.counter_d;
-        for (size_t j = 0; j <= nm; ++j)
-            g.args->prefix[j] = prefix[j];
     }
 #undef CKB
+    const msosm_status s = batch_plan(b);
+    if (s != MSOSM_OK) {
+        batch_release(b);
+        return s;
+    }
     *out = b;
     return MSOSM_OK;
 }
@@ -1420,6 +1457,11 @@ msosm_status msosm_batch_filter(msosm_batch *b, const void *const *inputs, int i
     for (const msosm_dedisp *d : b->h)
         if (check_outputs(d) != MSOSM_OK)
             return MSOSM_ERR_STATE;
+    if (batch_stale(b)) {
+        const msosm_status st = batch_plan(b);
+        if (st != MSOSM_OK)
+            return st;
+    }
     // handles outside every group: their whole call, one after another
     for (int i : b->alone) {
         msosm_status st = filter_block(b->h[i], inputs[i], kind);
