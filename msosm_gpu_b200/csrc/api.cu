@@ -15,6 +15,7 @@
 
 #include <cuda_runtime.h>
 
+#include "host_blocks.hpp"
 #include "host_prepare.hpp"
 #include "kernels.hpp"
 #include "tc_layout.hpp"
@@ -73,10 +74,13 @@ bool is_device_ptr(const void *p)
     return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
 }
 
-// The device address of page-locked host memory, null for any other
+// The device address of n values of host memory that lie in one block of
+// msosm_host_alloc; null for any other memory
 template <typename T>
-T *mapped_host(T *p)
+T *mapped_host(T *p, size_t n)
 {
+    if (!host_blocks().covers(p, n * sizeof(T)))
+        return nullptr;
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         cudaGetLastError();
@@ -1684,8 +1688,8 @@ msosm_status msosm_dedisp_get_profiles(msosm_dedisp *d, float *out)
     if (!d->fold)
         return fail(MSOSM_ERR_STATE, "fold not configured (msosm_dedisp_fold_init)");
     const size_t n = (size_t)d->D * d->nbins;
-    // page-locked memory is written by the kernel itself
-    float *direct = mapped_host(out);
+    // the kernel writes to page-locked memory of known extent itself
+    float *direct = mapped_host(out, n);
     CK(launch_fold_readout(d->acc_main, n, d->out_scale, direct ? direct : d->prof_out, d->stream));
     if (!direct)
         CK(cudaMemcpyAsync(out, d->prof_out, sizeof(float) * n, cudaMemcpyDeviceToHost, d->stream));

@@ -33,10 +33,18 @@
 
 #include <cuda_runtime.h>
 
+#include "host_blocks.hpp"
 #include "host_prepare.hpp"
 #include "kernels.hpp"
 
 using namespace msosm;
+
+// (never destroyed: blocks may be freed while the process ends)
+HostBlocks &msosm::host_blocks()
+{
+    static HostBlocks *const blocks = new HostBlocks;
+    return *blocks;
+}
 
 namespace {
 
@@ -370,6 +378,13 @@ msosm_status msosm_host_alloc(size_t bytes, int pinned, void **out)
             *out = nullptr;
             return sim_cuda_fail(e, "cudaMallocHost");
         }
+        try {
+            host_blocks().add(*out, bytes ? bytes : 1);
+        } catch (const std::bad_alloc &) {
+            cudaFreeHost(*out);
+            *out = nullptr;
+            return sim_fail(MSOSM_ERR_OOM, "host allocation");
+        }
         return MSOSM_OK;
     }
     *out = std::malloc(bytes ? bytes : 1);
@@ -381,6 +396,7 @@ msosm_status msosm_host_free(void *p, int pinned)
     if (!p)
         return MSOSM_OK;
     if (pinned) {
+        host_blocks().remove(p);
         cudaError_t e = cudaFreeHost(p);
         return e == cudaSuccess ? MSOSM_OK : sim_cuda_fail(e, "cudaFreeHost");
     }
