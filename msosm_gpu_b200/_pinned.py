@@ -14,6 +14,7 @@ import threading
 
 import numpy as np
 
+GRAIN = 64 << 10       # block sizes are multiples of this
 MIN_BYTES = 32 << 10   # below, the driver's staging costs no more
 MAX_BYTES = 32 << 20
 POOL_BYTES = 128 << 20
@@ -64,7 +65,7 @@ def empty(shape, dtype) -> np.ndarray:
     shape = (int(shape),) if np.isscalar(shape) else tuple(int(s) for s in shape)
     nbytes = int(np.prod(shape)) * np.dtype(dtype).itemsize
     if MIN_BYTES <= nbytes <= MAX_BYTES:
-        size = 1 << (nbytes - 1).bit_length()
+        size = -(-nbytes // GRAIN) * GRAIN
         address = _take(size)
         if address is not None:
             return np.asarray(_Block(address, size, shape, dtype))
