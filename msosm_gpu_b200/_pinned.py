@@ -32,7 +32,8 @@ def _take(size: int):
         if _free.get(size):
             return _free[size].pop()
         while _total + size > POOL_BYTES:
-            other = next((s for s, b in _free.items() if b), None)
+            # (a snapshot: an array collected meanwhile may add a size)
+            other = next((s for s, b in list(_free.items()) if b), None)
             if other is None:
                 return None
             lib().msosm_host_free(ctypes.c_void_p(_free[other].pop()), 1)

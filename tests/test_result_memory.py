@@ -1,4 +1,5 @@
-"""The pool of page-locked blocks behind result arrays: block sizes."""
+"""The pool of page-locked blocks behind result arrays: block sizes, and arrays collected in the
+middle of its work."""
 import ctypes
 import gc
 
@@ -36,3 +37,21 @@ def fake(monkeypatch):
 def test_block_sizes_follow_the_request(fake):
     a = _pinned.empty((1 << 17) + 1, np.uint32)  # a series with its trailing element: not twice the memory
     assert _pinned._total <= a.nbytes + _pinned.GRAIN
+
+
+def test_array_collected_while_room_is_made(fake, monkeypatch):
+    """Making room walks the waiting blocks; an array of a new size collected
+    just then comes back to the pool in the middle of the walk."""
+    monkeypatch.setattr(_pinned, "POOL_BYTES", 1 << 20)
+    held = [_pinned.empty(3 * _pinned.GRAIN, np.uint8)]
+
+    class Collected(list):
+        def __bool__(self):
+            held.clear()
+            gc.collect()
+            return len(self) > 0
+    keep = _pinned.empty(1 << 18, np.uint8)
+    _pinned._free.setdefault(_pinned.GRAIN, Collected())
+    _pinned._free[2 * _pinned.GRAIN] = Collected()
+    big = _pinned.empty(10 << 16, np.uint8)
+    assert big.size == 10 << 16 and keep.size == 1 << 18 and not held
