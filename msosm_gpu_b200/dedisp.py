@@ -166,14 +166,21 @@ class Dedisperser:
         elements the reference layout (trailing zero element) is filled."""
         n = self.numDMs * self.block_samples + 1
         if dtype == np.complex64:
-            buf = out if out is not None else _pinned.empty(n, np.complex64)
-            assert buf.dtype == np.complex64 and buf.size == n and buf.flags.c_contiguous
-            check(lib().msosm_dedisp_get_output_c64(self._h, buf.ctypes.data))
-            return buf if out is not None else buf[:-1].reshape(self.numDMs, self.block_samples)
-        buf = out if out is not None else _pinned.empty((n, 2), np.uint16)
-        assert buf.dtype == np.uint16 and buf.size == 2 * n and buf.flags.c_contiguous
-        check(lib().msosm_dedisp_get_output_uint16(self._h, buf.ctypes.data))
-        return buf if out is not None else buf[:-1].reshape(self.numDMs, self.block_samples, 2)
+            def read(p):
+                check(lib().msosm_dedisp_get_output_c64(self._h, p))
+            if out is None:
+                return _pinned.fetch(n, np.complex64, read)[:-1].reshape(self.numDMs, self.block_samples)
+            assert out.dtype == np.complex64 and out.size == n and out.flags.c_contiguous
+            read(out.ctypes.data)
+            return out
+
+        def read(p):
+            check(lib().msosm_dedisp_get_output_uint16(self._h, p))
+        if out is None:
+            return _pinned.fetch((n, 2), np.uint16, read)[:-1].reshape(self.numDMs, self.block_samples, 2)
+        assert out.dtype == np.uint16 and out.size == 2 * n and out.flags.c_contiguous
+        read(out.ctypes.data)
+        return out
 
     def output_device_ptr(self) -> int:
         p = ctypes.c_void_p()
@@ -191,9 +198,8 @@ class Dedisperser:
         self.folding = True
 
     def get_profiles(self) -> np.ndarray:
-        out = _pinned.empty((self.numDMs, self.time_bin), np.float32)
-        check(lib().msosm_dedisp_get_profiles(self._h, out.ctypes.data))
-        return out
+        return _pinned.fetch((self.numDMs, self.time_bin), np.float32,
+                             lambda p: check(lib().msosm_dedisp_get_profiles(self._h, p)))
 
     def folded_periods(self) -> int:
         n = ctypes.c_ulonglong()

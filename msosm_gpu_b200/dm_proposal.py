@@ -68,9 +68,13 @@ class DMProposalNet:
     def gradient(self, x, label, target, want_grad: bool = False):
         B = x.shape[0]
         loss = ctypes.c_float()
-        g = _pinned.empty(self.n_params, np.float32) if want_grad else None
-        check(lib().msosm_cnn_gradient(self._h, _ptr(x), _ptr(label), _ptr(target), B, ctypes.byref(loss),
-                                       None if g is None else g.ctypes.data))
+
+        def read(p):
+            check(lib().msosm_cnn_gradient(self._h, _ptr(x), _ptr(label), _ptr(target), B, ctypes.byref(loss), p))
+        if not want_grad:
+            read(None)
+            return float(loss.value), None
+        g = _pinned.fetch(self.n_params, np.float32, read)
         return float(loss.value), g
 
     def step(self, x, label, target, lr: float) -> float:
