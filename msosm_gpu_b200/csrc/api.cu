@@ -971,17 +971,15 @@ static msosm_status fold_prepare(msosm_dedisp *d, int sb, FoldArgs &fa)
     const bool smem = prof_in_smem(d);
     // the first block range that reaches into the pending period
     fa.pend_row = d->R;
-    if (n > 0 && d->spans[n - 1].dest == 2) {
-        if (d->large) {
-            fa.pend_row = d->R - 1;  // the last rows' share of the spans
-        } else {
-            const int bps = blocks_per_step(d);
-            const long long units = (d->count + bps - 1) / bps;
-            int r = d->R - 1;
-            while (r > 0 && (long long)bps * (units * r / d->R) * (long long)d->M > d->spans[n - 1].a)
-                --r;
-            fa.pend_row = r;
-        }
+    if (d->large) {
+        fa.pend_row = fold_direct_pend_row(d->bpt, d->R, d->D, (long long)d->count * (long long)d->M, d->spans.data(), n);
+    } else if (n > 0 && d->spans[n - 1].dest == 2) {
+        const int bps = blocks_per_step(d);
+        const long long units = (d->count + bps - 1) / bps;
+        int r = d->R - 1;
+        while (r > 0 && (long long)bps * (units * r / d->R) * (long long)d->M > d->spans[n - 1].a)
+            --r;
+        fa.pend_row = r;
     }
     if (!smem && !d->large) {
         // the kernel adds to its partial rows in memory
@@ -1607,7 +1605,7 @@ msosm_status msosm_dedisp_fold_init(msosm_dedisp *d, float period, float fs, uns
             return cuda_fail(e, "plan_grid");
         }
     } else {
-        d->R = fold_direct_rows(d->nbins, d->bpt, d->D, d->span_cap);
+        d->R = fold_direct_rows(d->nbins, d->bpt, d->D, d->span_cap, (long long)d->count * (long long)d->M);
     }
     d->fold = false;
     size_t &tot = d->device_bytes;
@@ -1820,7 +1818,7 @@ msosm_status msosm_fold_create(float period, float fs, unsigned long size, unsig
     f->bpt = nb == f->ps ? 1 : (int)(f->ps / nb);
     f->out_scale = nb == f->ps ? 1.0 : 1.0 / (double)f->bpt;
     f->span_cap = (int)(size / f->ps) + 8;
-    f->R = fold_direct_rows(f->nbins, f->bpt, 1, f->span_cap);
+    f->R = fold_direct_rows(f->nbins, f->bpt, 1, f->span_cap, (long long)size);
     size_t tot = 0;
 #define CKF(call)                                                                                      \
     do {                                                                                               \
@@ -1975,7 +1973,7 @@ msosm_status msosm_fold_data(msosm_fold *f)
     a.span_cap = 0;
     a.inv_bpt = 1.0f / (float)f->bpt;
     a.g_shift = 0;
-    a.pend_row = n > 0 && f->spans[n - 1].dest == 2 ? f->R - 1 : f->R;
+    a.pend_row = fold_direct_pend_row(f->bpt, f->R, 1, (long long)f->size, f->spans.data(), n);
     CK(launch_fold_direct(f->I, (long long)f->size, f->R, a, 1, f->stream));
     CK(launch_fold_reduce(f->part_main, f->part_pend, 1, f->R, f->nbins, a.pend_row, nullptr, f->acc_main, f->acc_pend,
                           f->stream));

@@ -22,6 +22,7 @@
 #include "kernels.hpp"
 #include "tc_layout.hpp"
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -127,6 +128,9 @@ __global__ void intensity_kernel(const float2 *__restrict__ a, const float2 *__r
 // lanes per output bin adds the bin's samples of every span of row r's share
 // [nspans r / R, nspans (r + 1) / R) and writes them to partial row r (the main
 // and the pending sums); trial d = blockIdx.z folds I[d n ...] into rows r D + d.
+// For bins of up to 1024 samples, and up to 4096 where the chunk fills a
+// thousand of them (fold_wide): a lane adds at most 128 samples of a span (32
+// to an accumulator) and eight spans in FP32, more spans in FP64.
 // Bound by latency: a lane's loads are independent, and blocks and rows are
 // cut so that about 1200 blocks share the chunk (fold_direct_rows).  At 84
 // periods of 49600 samples and 1024 bins the staged form (2048 samples to
@@ -138,10 +142,18 @@ __global__ void __launch_bounds__(256) fold_direct_kernel(const float *__restric
     const int G = 1 << f.g_shift, l = threadIdx.x & (G - 1);
     const int bin = (int)blockIdx.x * (256 >> f.g_shift) + (int)(threadIdx.x >> f.g_shift);
     const int s0 = (int)((long long)f.nspans * r / R), s1 = (int)((long long)f.nspans * (r + 1) / R);
+    // the sums of eight spans in FP32, more in FP64
+    const bool many = s1 - s0 > 8, with_pend = r >= f.pend_row;
     float main = 0.f, pend = 0.f;
+    double mains = 0.0, pends = 0.0;
     if (bin < f.nbins) {
         const long long p0 = (long long)bin * f.bpt;
         for (int s = s0; s < s1; ++s) {
+            if (many && ((s - s0) & 7) == 0) {
+                mains += (double)main;
+                pends += (double)pend;
+                main = pend = 0.f;
+            }
             const int dest = f.span_dest[s];
             if (dest == 0)
                 continue;
@@ -170,15 +182,134 @@ __global__ void __launch_bounds__(256) fold_direct_kernel(const float *__restric
                 pend += sum;
         }
     }
-    for (int o = G >> 1; o > 0; o >>= 1) {
-        main += __shfl_xor_sync(0xffffffffu, main, o);
-        pend += __shfl_xor_sync(0xffffffffu, pend, o);
+    if (many) {
+        mains += (double)main;
+        pends += (double)pend;
+        for (int o = G >> 1; o > 0; o >>= 1) {
+            mains += __shfl_xor_sync(0xffffffffu, mains, o);
+            if (with_pend)
+                pends += __shfl_xor_sync(0xffffffffu, pends, o);
+        }
+        main = (float)mains;
+        pend = (float)pends;
+    } else {
+        for (int o = G >> 1; o > 0; o >>= 1) {
+            main += __shfl_xor_sync(0xffffffffu, main, o);
+            if (with_pend)
+                pend += __shfl_xor_sync(0xffffffffu, pend, o);
+        }
     }
     if (bin < f.nbins && l == 0) {
         const size_t at = ((size_t)r * D + d) * f.nbins + bin;
         f.part_main[at] = main;
-        if (r >= f.pend_row)
+        if (with_pend)
             f.part_pend[at] = pend;
+    }
+}
+
+// The same for long bins (fold_wide): partial row r takes the samples [n r / R, n (r + 1) / R) whatever spans they lie in, and the whole
+// block adds the samples of a bin.  With few long bins the form above has
+// nothing to share out: at 4 bins of 2.8 million samples one span's worth of
+// lanes did everything, 2.4 ms a call of 2^20 samples (37 us here, of which 35 are
+// the call and its readout).
+// A thread adds at most 64 samples in FP32 (16 to an accumulator); those sums,
+// the threads and the spans in FP64.
+// A row shorter than a period touches the bins from that of its first sample
+// on, at most len / bpt + 3 of them; the others are zero.
+__global__ void __launch_bounds__(256) fold_wide_kernel(const float *__restrict__ I, long long n, FoldArgs f)
+{
+    constexpr int W = 8, GROUP = 16;  // warps; bins between two barriers
+    __shared__ double sums[2][GROUP][W];
+    const int r = blockIdx.x, R = gridDim.x, d = blockIdx.y, D = gridDim.y;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long t0 = n * r / R, t1 = n * (r + 1) / R;
+    I += (size_t)d * n;
+    const size_t row = ((size_t)r * D + d) * f.nbins;
+    const bool with_pend = r >= f.pend_row;
+    for (int i = threadIdx.x; i < f.nbins; i += 256) {
+        f.part_main[row + i] = 0.f;
+        if (with_pend)
+            f.part_pend[row + i] = 0.f;
+    }
+    // the spans that reach into the row
+    int lo = 0, s1 = f.nspans;
+    while (lo < s1) {
+        const int mid = (lo + s1) >> 1;
+        if (f.span_b[mid] <= t0)
+            lo = mid + 1;
+        else
+            s1 = mid;
+    }
+    const int s0 = lo;
+    if (s0 >= f.nspans || f.span_a[s0] >= t1)
+        return;
+    for (s1 = s0 + 1; s1 < f.nspans && f.span_a[s1] < t1;)
+        ++s1;
+    const long long a0 = f.span_a[s0];
+    const long long first = (f.span_phase0[s0] + (t0 > a0 ? t0 - a0 : 0)) / f.bpt;
+    const long long most = (t1 - t0) / f.bpt + 3;
+    const int b0 = first < f.nbins ? (int)first : 0, count = most < f.nbins ? (int)most : f.nbins;
+    for (int c0 = 0; c0 < count; c0 += GROUP) {
+        const int cn = min(GROUP, count - c0);
+        __syncthreads();  // the zeroes are written, the last group's sums read
+        for (int c = 0; c < cn; ++c) {
+            int bin = b0 + c0 + c;
+            bin -= bin >= f.nbins ? f.nbins : 0;
+            const long long p0 = (long long)bin * f.bpt;
+            double main = 0.0, pend = 0.0;
+            for (int s = s0; s < s1; ++s) {
+                const int dest = f.span_dest[s];
+                if (dest == 0)
+                    continue;
+                // samples [x, y) of the chunk: this bin, this span, this row
+                const long long off = f.span_a[s] - f.span_phase0[s];
+                const long long x = max(max(f.span_a[s], t0), off + p0);
+                const long long y = min(min(f.span_b[s], t1), off + p0 + f.bpt);
+                double sum = 0.0;
+                for (long long q = x; q < y; q += 64 * 256) {
+                    const int m = (int)min(y - q, 64ll * 256);
+                    const float *src = I + q;
+                    float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
+                    int p = threadIdx.x;
+                    for (; p + 3 * 256 < m; p += 4 * 256) {
+                        v0 += src[p];
+                        v1 += src[p + 256];
+                        v2 += src[p + 2 * 256];
+                        v3 += src[p + 3 * 256];
+                    }
+                    if (p < m)
+                        v0 += src[p];
+                    if (p + 256 < m)
+                        v1 += src[p + 256];
+                    if (p + 2 * 256 < m)
+                        v2 += src[p + 2 * 256];
+                    sum += (double)((v0 + v1) + (v2 + v3));
+                }
+                if (dest == 1)
+                    main += sum;
+                else
+                    pend += sum;
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                main += __shfl_xor_sync(0xffffffffu, main, o);
+                pend += __shfl_xor_sync(0xffffffffu, pend, o);
+            }
+            if (lane == 0) {
+                sums[0][c][warp] = main;
+                sums[1][c][warp] = pend;
+            }
+        }
+        __syncthreads();
+        const int c = threadIdx.x >> 1, which = threadIdx.x & 1;
+        if (c < cn && (which == 0 || with_pend)) {
+            double v = 0.0;
+#pragma unroll
+            for (int w = 0; w < W; ++w)
+                v += sums[which][c][w];
+            int bin = b0 + c0 + c;
+            bin -= bin >= f.nbins ? f.nbins : 0;
+            (which ? f.part_pend : f.part_main)[row + bin] = (float)v;
+        }
     }
 }
 
@@ -617,16 +748,45 @@ static int direct_tiles(int nbins, int bpt)
     return (nbins + per - 1) / per;
 }
 
-int fold_direct_rows(int nbins, int bpt, int trials, int max_spans)
+// Whether a call of n samples takes the second form.  A warp of the first form
+// adds one bin of one span: with fewer than about 1024 of those the chunk waits
+// for them.  2^22 samples, bins of 20000: 104 us a call in the first form, 54 in
+// the second; 2^20 of 10937: 65 and 40; 2^22 of 3100 (1353 warps): 42 and 50.
+static bool fold_wide(int bpt, int trials, long long n)
 {
+    return bpt > 4096 || (bpt > 1024 && n / bpt * trials < 1024);
+}
+
+int fold_direct_rows(int nbins, int bpt, int trials, int max_spans, long long n)
+{
+    if (fold_wide(bpt, trials, n)) {
+        // rows of 4096 samples, 1200 blocks in all at most; 2^24 partial sums
+        const long long R = std::min(std::min(n / 4096, 1200ll / trials), (1ll << 24) / ((long long)nbins * trials));
+        return (int)std::max(R, 1ll);
+    }
     const long long tiles = (long long)direct_tiles(nbins, bpt) * trials;
     const long long R = 1200 / tiles;
     return (int)(R < 1 ? 1 : (R > max_spans ? max_spans : R));
 }
 
+int fold_direct_pend_row(int bpt, int R, int trials, long long n, const FoldSpan *spans, int nspans)
+{
+    if (nspans == 0 || spans[nspans - 1].dest != 2)
+        return R;
+    int r = R - 1;  // the last share of the spans
+    if (fold_wide(bpt, trials, n))  // the row the period begins in
+        while (r > 0 && n * r / R > spans[nspans - 1].a)
+            --r;
+    return r;
+}
+
 cudaError_t launch_fold_direct(const float *I, long long n, int R, const FoldArgs &args, int trials, cudaStream_t st)
 {
     FoldArgs f = args;
+    if (fold_wide(f.bpt, trials, n)) {
+        fold_wide_kernel<<<dim3((unsigned)R, (unsigned)trials), 256, 0, st>>>(I, n, f);
+        return cudaGetLastError();
+    }
     f.g_shift = direct_g_shift(f.bpt);
     fold_direct_kernel<<<dim3((unsigned)direct_tiles(f.nbins, f.bpt), (unsigned)R, (unsigned)trials), 256, 0, st>>>(I, n,
                                                                                                                    f);

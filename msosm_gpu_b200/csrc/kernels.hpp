@@ -158,8 +158,10 @@ cudaError_t launch_encode_u16(const float2 *src, uint32_t *dst, size_t n, cudaSt
 // sqrt(|a|^2 + |b|^2) (b may be null)
 cudaError_t launch_intensity(const float2 *a, const float2 *b, float *out, size_t n, cudaStream_t st);
 // fold n intensities of each trial into R partial rows per trial (fold.part_main / part_pend
-// [R][trials][nbins]); the rows to use for at most max_spans spans a call
-int fold_direct_rows(int nbins, int bpt, int trials, int max_spans);
+// [R][trials][nbins]); the rows to use for at most max_spans spans a call of n samples, and the
+// first of them that holds pending samples (FoldArgs::pend_row)
+int fold_direct_rows(int nbins, int bpt, int trials, int max_spans, long long n);
+int fold_direct_pend_row(int bpt, int R, int trials, long long n, const FoldSpan *spans, int nspans);
 cudaError_t launch_fold_direct(const float *I, long long n, int R, const FoldArgs &f, int trials, cudaStream_t st);
 
 // ---- tensor-core (tcgen05) dedispersion, 4096-, 8192- and 16384-point transforms (tc_dedisp.cu)
