@@ -315,6 +315,35 @@ size_t fold_smem(const msosm_dedisp *d)
     return d->fold ? fold_smem_bytes(d->nbins, d->win_cap, prof_in_smem(d)) : 0;
 }
 
+// The fewest block ranges a trial is cut into.  For precision:
+//  - f16 operands are scaled by one power of two per work item, so a strong
+//    burst takes bits from every block of its range.  About eight items per
+//    resident CTA keep that to an eighth of a call or less (148 trials at 8192
+//    points, one block 100 dB above the noise: error of the blocks long after
+//    it 1.1e-3, in one range per trial 4.6e-3);
+//  - a bin's sum over a range is FP32: p periods of equal size leave a relative
+//    error of about 2^-25 sqrt(p / 3), R ranges of P / R periods 2^-25
+//    sqrt(P / 3) / R.  R >= sqrt(P / 12) keeps it below 6e-8, small against the
+//    transforms' own 3-4e-7 (1353 periods in one range: 5.7e-7), up to eight
+//    items per 8192 samples in flight on an SM: beyond those an item is mostly
+//    its own filter and profile rows.
+// And for the FP32 kernel's CTAs, which do not run equally fast and take items
+// from a counter: eight items each, while an item keeps 24 steps (592 trials of
+// 2^21 samples at 4096 points: 5.92 ms with one range, 6.41 with two, 5.71 with
+// four).
+long long min_ranges(const msosm_dedisp *d, long long units, long long resident, int sms)
+{
+    const long long even = d->tc ? 1 : std::min((8 * resident + d->D - 1) / d->D, units / 24);
+    const long long in_flight = d->tc ? resident : (long long)sms * std::max(1ul, 8192 / d->M);
+    const long long eight = (8 * in_flight + d->D - 1) / d->D;
+    if (d->tc && !d->tc_bf16)
+        return eight;
+    if (!d->fold)
+        return even;
+    const double periods = (double)d->count * (double)d->M / (double)d->ps;
+    return std::max(even, std::min(eight, (long long)std::ceil(std::sqrt(periods / 12.0))));
+}
+
 // Block ranges per trial and the persistent grid of the dedispersion kernel.
 // A work item is one (block range, trial); the grid strides over the items.
 // The ranges are chosen so that the items fill whole waves of the resident
@@ -345,12 +374,13 @@ cudaError_t plan_grid(msosm_dedisp *d)
     const int bps = blocks_per_step(d);
     const long long units = (d->count + bps - 1) / bps;
     constexpr double kItemSteps = 1.5;
-    const long long r_max = std::max(1ll, std::min(units, 12 * resident / d->D + 1));
+    const long long r_min = std::max(1ll, std::min(units, min_ranges(d, units, resident, sms)));
+    const long long r_max = std::min(units, std::max(2 * r_min, 12 * resident / d->D + 1));
     double best = 0.0;
-    for (long long R = 1; R <= r_max; ++R) {
+    for (long long R = r_min; R <= r_max; ++R) {
         const long long waves = ((long long)d->D * R + resident - 1) / resident;
         const double cost = (double)waves * ((double)((units + R - 1) / R) + kItemSteps);
-        if (R == 1 || cost < best) {
+        if (R == r_min || cost < best) {
             best = cost;
             d->R = (int)R;
         }

@@ -207,7 +207,8 @@ __global__ void __launch_bounds__(256) fold_direct_kernel(const float *__restric
     }
 }
 
-// The same for long bins (fold_wide): partial row r takes the samples [n r / R, n (r + 1) / R) whatever spans they lie in, and the whole
+// The same for long bins (fold_wide): partial row r takes the samples
+// [n r / R, n (r + 1) / R) whatever spans they lie in, and the whole
 // block adds the samples of a bin.  With few long bins the form above has
 // nothing to share out: at 4 bins of 2.8 million samples one span's worth of
 // lanes did everything, 2.4 ms a call of 2^20 samples (37 us here, of which 35 are
