@@ -260,6 +260,21 @@ msosm_status upload_table(float2 **dst, int n, int sign, size_t &total, cudaStre
     return MSOSM_OK;
 }
 
+// The same with the stage-1 entries of the row passes behind it (kStage1):
+// exp(sign 2 pi i m r / 256) at n + 16 r + m
+msosm_status upload_row_table(float2 **dst, int n, int sign, size_t &total, cudaStream_t st)
+{
+    std::vector<float2> t = twiddle_table(n, sign);
+    const std::vector<float2> w = twiddle_table(kStage1Entries, sign);
+    for (int r = 0; r < 16; ++r)
+        for (int m = 0; m < 16; ++m)
+            t.push_back(w[m * r]);
+    CK(dalloc(dst, t.size(), total));
+    CK(cudaMemcpyAsync(*dst, t.data(), sizeof(float2) * t.size(), cudaMemcpyHostToDevice, st));
+    CK(cudaStreamSynchronize(st));
+    return MSOSM_OK;
+}
+
 // H of every trial on the device: H_ref * scale into H[D][N]
 msosm_status design_filters(int log2n, const std::vector<ChirpParams> &cp, float scale, int sign,
                             const float2 *tw_inv_m, const float2 *tw_fwd, float2 *H, cudaStream_t st)
@@ -427,7 +442,7 @@ int ChirpIdft::init(int log2m_, cudaStream_t st)
         large_split(log2m, m1l, m2l);
         s = upload_table(&tw1, 1 << m1l, -1, tot, st);
         if (s == MSOSM_OK)
-            s = upload_table(&tw2, 1 << m2l, -1, tot, st);
+            s = upload_row_table(&tw2, 1 << m2l, -1, tot, st);
     } else {
         s = upload_table(&tw1, 1 << log2m, -1, tot, st);
     }
@@ -515,7 +530,7 @@ msosm_status design_filters_large(int log2n, const std::vector<ChirpParams> &cp,
     if (s == MSOSM_OK)
         s = upload_table(&twn1, 1 << n1l, -1, tot, st);
     if (s == MSOSM_OK)
-        s = upload_table(&twn2, 1 << n2l, -1, tot, st);
+        s = upload_row_table(&twn2, 1 << n2l, -1, tot, st);
     if (s == MSOSM_OK) {
         for (size_t i = 0; i < cp.size() && e == cudaSuccess; ++i) {
             e = idft.run(cp[i], sign, P, N, st);
@@ -875,8 +890,8 @@ msosm_status msosm_dedisp_create(const float *bw, const float *dm, const float *
     } else {
         if ((s = upload_table(&d->tw1f, 1 << d->log2n1, -1, tot, d->stream)) != MSOSM_OK ||
             (s = upload_table(&d->tw1i, 1 << d->log2n1, +1, tot, d->stream)) != MSOSM_OK ||
-            (s = upload_table(&d->tw2f, 1 << d->log2n2, -1, tot, d->stream)) != MSOSM_OK ||
-            (s = upload_table(&d->tw2i, 1 << d->log2n2, +1, tot, d->stream)) != MSOSM_OK) {
+            (s = upload_row_table(&d->tw2f, 1 << d->log2n2, -1, tot, d->stream)) != MSOSM_OK ||
+            (s = upload_row_table(&d->tw2i, 1 << d->log2n2, +1, tot, d->stream)) != MSOSM_OK) {
             release(d);
             return s;
         }

@@ -219,8 +219,16 @@ __device__ __forceinline__ void twiddle_powers(float2 (&w)[16], const float2 *__
     }
 }
 
+// Where a stage's twiddles come from.  kPowers: two table reads and products of
+// them (twiddle_powers).  kTable: all R - 1 from the table, for callers whose
+// lanes share the index (the column passes of the four-step transforms: one
+// transaction a read, and no product's rounding).  kStage1: those of stage 1,
+// where that has radix 16, from 256 entries behind the table, W_256^(m r) at
+// N + 16 r + m (16 values of m, one line a read); the later stages by powers.
+enum TwiddleSource { kPowers, kTable, kStage1 };
+
 // Twiddle + butterflies of stage S (tw: table exp(SIGN 2 pi i e / N), e < N).
-template <int LOG2N, int S, int SIGN>
+template <int LOG2N, int S, int SIGN, TwiddleSource TW = kPowers>
 __device__ __forceinline__ void stage_compute(float2 (&v)[16], int tid, const float2 *__restrict__ tw)
 {
     using F = FftShape<LOG2N>;
@@ -232,7 +240,13 @@ __device__ __forceinline__ void stage_compute(float2 (&v)[16], int tid, const fl
             const int m = j & (NS - 1);
             constexpr int STEP = F::N / (NS * R);
             float2 w[16];
-            twiddle_powers<R>(w, tw, m * STEP, 4 * m * STEP);
+            if constexpr (TW == kTable || (TW == kStage1 && S == 1 && R == 16)) {
+#pragma unroll
+                for (int r = 1; r < R; ++r)
+                    w[r] = __ldg(TW == kTable ? tw + r * m * STEP : tw + F::N + 16 * r + m);
+            } else {
+                twiddle_powers<R>(w, tw, m * STEP, 4 * m * STEP);
+            }
 #pragma unroll
             for (int r = 1; r < R; ++r)
                 v[q * R + r] = cmul(v[q * R + r], w[r]);
@@ -286,7 +300,7 @@ __device__ __forceinline__ int last_out_index(int tid, int slot)
 // last-stage loads are done (no barrier after them): the caller must
 // synchronise before anything overwrites the buffer the last stage read,
 // buf[(NST-2)&1] with PINGPONG, buf0 otherwise.
-template <int LOG2N, int SIGN, bool PINGPONG, int S = 1>
+template <int LOG2N, int SIGN, bool PINGPONG, TwiddleSource TW = kPowers, int S = 1>
 __device__ __forceinline__ void run_stages(float2 (&v)[16], float2 *buf0, float2 *buf1, int tid,
                                            const float2 *__restrict__ tw, bool active = true)
 {
@@ -301,13 +315,13 @@ __device__ __forceinline__ void run_stages(float2 (&v)[16], float2 *buf0, float2
             if constexpr (!PINGPONG)
                 __syncthreads();
             if (active) {
-                stage_compute<LOG2N, S, SIGN>(v, tid, tw);
+                stage_compute<LOG2N, S, SIGN, TW>(v, tid, tw);
                 stage_store<LOG2N, S>(v, dst, tid);
             }
-            run_stages<LOG2N, SIGN, PINGPONG, S + 1>(v, buf0, buf1, tid, tw, active);
+            run_stages<LOG2N, SIGN, PINGPONG, TW, S + 1>(v, buf0, buf1, tid, tw, active);
         } else {
             if (active)
-                stage_compute<LOG2N, S, SIGN>(v, tid, tw);
+                stage_compute<LOG2N, S, SIGN, TW>(v, tid, tw);
         }
     }
 }

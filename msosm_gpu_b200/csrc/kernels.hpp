@@ -206,6 +206,8 @@ struct LargeColArgs {
     float *intensity;         // inverse: [d][count*M] or null
     int detect;
 };
+// entries behind a row table: exp(sign 2 pi i m r / 256) at 16 r + m
+constexpr int kStage1Entries = 256;
 struct LargeRowArgs {
     const float2 *in;         // forward: A
     float2 *out;              // inverse: B; design: permuted spectrum
@@ -217,7 +219,7 @@ struct LargeRowArgs {
     const uint16_t *delays;   // [d][N] permuted
     long long N;
     int log2n;
-    const float2 *tw2;        // exp(sign 2 pi i e / N2)
+    const float2 *tw2;        // exp(sign 2 pi i e / N2), then the stage-1 entries (kStage1Entries)
     const float2 *tw2i;       // mode 3: the inverse pass's table
 };
 void large_split(int log2n, int &log2n1, int &log2n2);

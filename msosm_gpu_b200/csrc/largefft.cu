@@ -15,7 +15,12 @@
 // Column passes run 16 or 32 columns per thread block (independent N1-point
 // block FFTs whose global reads and writes are rows of 16 or 32 elements); row
 // passes run one N2-point block FFT per thread block.  Twiddles W_N^e come
-// from sincospif of the exact float 2e/N and products of two or three of them.
+// from sincospif of the exact float 2e/N, at most one product of two of them.
+// The block FFTs' own twiddles are table values where a read is one
+// transaction: all of the column passes', whose lanes (columns) share the
+// index, and stage 1's of the row passes.  With products there too the column
+// passes of 256 points and more made a profile's error grow with their number
+// of stages (2^20 and 2^21 points: 6.3e-7 - 6.9e-7, now 4.6e-7 - 5.1e-7, at the same time).
 #include "chirp.cuh"
 #include "fft_smem.cuh"
 #include "kernels.hpp"
@@ -51,9 +56,8 @@ __device__ __forceinline__ float2 twiddle_n(int e, int log2n, float sign)
 // (last_out_index: slot q R + r holds m = q + r 16/R).  Seven sines and cosines and one
 // product per factor instead of sixteen sines and cosines: those, with the 64-bit
 // indices, were most of the column pass's instructions (54 us for 32 windows
-// of 2^18 points).  One call at 2^18: 144.6 us, with sixteen 159.3, with five and up to
-// three products 143.3, but there the profile's error against FP64 grew from 6.0e-7
-// to 6.1e-7; with one product it is 6.0e-7 as with sixteen.
+// of 2^18 points).  One call at 2^18: 144.6 us, with sixteen 159.3.  The error of
+// a series against FP64 is 1 % larger than with sixteen, that of a profile the same.
 template <int LOG2L>
 __device__ __forceinline__ void twiddle_outputs(float2 (&v)[16], int a, int j, int log2n, float sign)
 {
@@ -129,7 +133,7 @@ __global__ void __launch_bounds__(ColShape<LOG2N1>::THREADS, ColShape<LOG2N1>::B
     }
     dft16<-1>(v);
     stage_store<LOG2N1, 0>(v, buf, j);
-    run_stages<LOG2N1, -1, false>(v, buf, buf, j, a.tw1);
+    run_stages<LOG2N1, -1, false, kTable>(v, buf, buf, j, a.tw1);
     twiddle_outputs<LOG2N1>(v, n2, j, a.log2n, -1.f);
     float2 *out = a.out + (size_t)w * a.N + n2;
 #pragma unroll
@@ -180,7 +184,7 @@ __global__ void __launch_bounds__(FftShape<LOG2N2>::T, FftShape<LOG2N2>::T >= 10
             v[r] = in[j + r * T2];
         dft16<-1>(v);
         stage_store<LOG2N2, 0>(v, smem, j);
-        run_stages<LOG2N2, -1, false>(v, smem, smem, j, a.tw2);
+        run_stages<LOG2N2, -1, false, kStage1>(v, smem, smem, j, a.tw2);
     }
     if constexpr (MODE == 3) {
         // the slots hold k2 = j + m T2, the inverse's inputs in another order
@@ -199,7 +203,7 @@ __global__ void __launch_bounds__(FftShape<LOG2N2>::T, FftShape<LOG2N2>::T >= 10
         dft16<+1>(v);
         stage_store<LOG2N2, 0>(v, smem, j);
         // (the twiddles of the two directions are conjugate tables)
-        run_stages<LOG2N2, +1, false>(v, smem, smem, j, MODE == 3 ? a.tw2i : a.tw2);
+        run_stages<LOG2N2, +1, false, kStage1>(v, smem, smem, j, MODE == 3 ? a.tw2i : a.tw2);
         twiddle_outputs<LOG2N2>(v, k1, j, a.log2n, +1.f);
         float2 *out = a.out + ((size_t)d * a.count + w) * N + row;
 #pragma unroll
@@ -238,7 +242,7 @@ __global__ void __launch_bounds__(ColShape<LOG2N1>::THREADS, ColShape<LOG2N1>::B
         v[r] = in[(j + r * T1) * N2 + n2];
     dft16<+1>(v);
     stage_store<LOG2N1, 0>(v, buf, j);
-    run_stages<LOG2N1, +1, false>(v, buf, buf, j, a.tw1);
+    run_stages<LOG2N1, +1, false, kTable>(v, buf, buf, j, a.tw1);
     const size_t base = ((size_t)d * a.count + w) * M;
 #pragma unroll
     for (int slot = 0; slot < 16; ++slot) {
