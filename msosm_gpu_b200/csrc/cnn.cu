@@ -387,22 +387,25 @@ struct WgradRows {
 };
 
 // Sum of the groups' rows of every layer (blockIdx.y) in one launch after the
-// backward pass.  Eight slices of the rows per value, added in order.  Bound by
+// backward pass.  Eight slices of the rows per value, added in order, in FP64:
+// in FP32 these few additions of nearly whole sums were most of a weight
+// gradient's rounding (1.3e-7 of its size, 0.9e-7 now, last layer of the
+// defaults).  Bound by
 // latency: a launch per layer, each between two convolutions, took 5 - 7 us (a
 // gradient of 256 samples and four layers 459 us, with one launch 442).
 __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const __grid_constant__ WgradRows rows)
 {
-    __shared__ float sums[8][32];
+    __shared__ double sums[8][32];
     const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5, l = blockIdx.y, groups = rows.groups[l];
     const long long i = (long long)blockIdx.x * 32 + lane, n = rows.values[l];
     if ((long long)blockIdx.x * 32 >= n)
         return;
     const float *__restrict__ part = rows.part + rows.offset[l];
-    float s = 0.f;
+    double s = 0.0;
     if (i < n) {
 #pragma unroll 4
         for (int g = sl; g < groups; g += 8)
-            s += part[(size_t)g * n + i];
+            s += (double)part[(size_t)g * n + i];
     }
     sums[sl][lane] = s;
     __syncthreads();
@@ -410,7 +413,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const __grid_constant
 #pragma unroll
         for (int k = 1; k < 8; ++k)
             s += sums[k][lane];
-        rows.grad[rows.out[l] + i] = s;
+        rows.grad[rows.out[l] + i] = (float)s;
     }
 }
 
@@ -501,18 +504,20 @@ __global__ void __launch_bounds__(1024) pool_heads_kernel(const float *__restric
     __syncthreads();
     if (threadIdx.x >= 32)
         return;
-    float lg = 0.f, of = 0.f;
+    // (FP64: a few hundred operations of one warp; the terms cancel, and what
+    // their rounding leaves goes into the loss and every gradient)
+    double lg = 0.0, of = 0.0;
     for (int c = lane; c < C; c += 32) {
-        lg = fmaf(hs[c], __bfloat162float(wd[c]), lg);
-        of = fmaf(hs[c], __bfloat162float(wr[c]), of);
+        lg = fma((double)hs[c], (double)__bfloat162float(wd[c]), lg);
+        of = fma((double)hs[c], (double)__bfloat162float(wr[c]), of);
     }
     for (int o = 16; o > 0; o >>= 1) {
         lg += __shfl_xor_sync(0xffffffffu, lg, o);
         of += __shfl_xor_sync(0xffffffffu, of, o);
     }
     if (lane == 0) {
-        logit[b] = lg + *bd;
-        offset[b] = of + *br;
+        logit[b] = (float)(lg + (double)*bd);
+        offset[b] = (float)(of + (double)*br);
     }
 }
 
