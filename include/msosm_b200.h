@@ -314,7 +314,7 @@ MSOSM_API msosm_status msosm_fold_get_shape(const msosm_fold *f, unsigned long *
 typedef struct msosm_timing {
     double forward_ms;  /* decode + forward FFT into the spectrum ring */
     double dedisp_ms;   /* fused gather x H, inverse FFT, discard, detect, fold */
-    double fold_ms;     /* fold bookkeeping: partial-row clears, ordered reduce, flush */
+    double fold_ms;     /* fold bookkeeping: span table, flush, ordered reduce */
     double h2d_ms;      /* host-to-device input staging (copy stream) */
     unsigned long long calls;           /* filter calls timed */
     unsigned long long kernel_launches; /* kernels of this library launched by those calls */

@@ -1276,7 +1276,8 @@ static msosm_status filter_block(msosm_dedisp *d, const void *input, InputKind k
     msosm_status st = call_begin(d, input, kind, ev, launches0, da, done);
     if (st != MSOSM_OK || done)
         return st;
-    // the partial-row clears and the flush above belong to the fold time;
+    // the fold's bookkeeping above (span table, flush, and the clears of
+    // profiles too long for shared memory) belongs to the fold time;
     // the dedispersion kernel is timed alone
     if (ev)
         CK(cudaEventRecord(ev->e[2], d->stream));
@@ -2003,7 +2004,7 @@ msosm_status msosm_fold_data(msosm_fold *f)
     int launched = 0;
     CK(launch_fold_begin(f->spans.data(), n, f->span_host, f->span_cap, f->span_a, f->span_b, f->span_p, f->span_dest,
                          flush, f->acc_main, f->acc_pend, (size_t)f->nbins, f->stream, &launched));
-    FoldArgs a;
+    FoldArgs a{};  // (the fields of the fused fold's shared memory stay unused)
     a.span_a = f->span_a;
     a.span_b = f->span_b;
     a.span_phase0 = f->span_p;
@@ -2011,13 +2012,8 @@ msosm_status msosm_fold_data(msosm_fold *f)
     a.nspans = n;
     a.bpt = f->bpt;
     a.nbins = f->nbins;
-    a.detect = 0;
     a.part_main = f->part_main;
     a.part_pend = f->part_pend;
-    a.smem_prof = 0;
-    a.span_cap = 0;
-    a.inv_bpt = 1.0f / (float)f->bpt;
-    a.g_shift = 0;
     a.pend_row = fold_direct_pend_row(f->bpt, f->R, 1, (long long)f->size, f->spans.data(), n);
     CK(launch_fold_direct(f->I, (long long)f->size, f->R, a, 1, f->stream));
     CK(launch_fold_reduce(f->part_main, f->part_pend, 1, f->R, f->nbins, a.pend_row, nullptr, f->acc_main, f->acc_pend,

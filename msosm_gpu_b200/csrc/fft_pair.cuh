@@ -1,4 +1,4 @@
-// fft_pair.cuh -- block-wide inverse/forward FFT of PAIRS of transforms on
+// fft_pair.cuh -- block-wide inverse FFT of PAIRS of transforms on
 // packed FP32 arithmetic (fma/add/mul .f32x2 of sm_100a).
 //
 // Radix 16 with one last stage of radix 2, 4 or 8 where the size needs it;
@@ -96,30 +96,27 @@ __device__ __forceinline__ c2 ctw(c2 v, float wx, float wy)
     return {pk(r.x * wx - i.x * wy, r.y * wx - i.y * wy), pk(r.x * wy + i.x * wx, r.y * wy + i.y * wx)};
 }
 
-template <int SIGN>
 __device__ __forceinline__ void dft4(c2 &x0, c2 &x1, c2 &x2, c2 &x3)
 {
     const c2 a = cadd(x0, x2), b = csub(x0, x2), c = cadd(x1, x3), e = csub(x1, x3);
     x0 = cadd(a, c);
     x2 = csub(a, c);
-    x1 = cadd_i<SIGN>(b, e);
-    x3 = cadd_i<-SIGN>(b, e);
+    x1 = cadd_i<+1>(b, e);
+    x3 = cadd_i<-1>(b, e);
 }
 
 // x[t] = X[4 t'] combinations of four values of which 1..3 still lack the
 // factor k1 (1 and 3) or k2 (2): a0, k1 u1, k2 u2, k1 u3
-template <int SIGN>
 __device__ __forceinline__ void dft4_scaled(c2 a0, c2 u1, c2 u2, c2 u3, float k1, float k2, c2 &x0, c2 &x1, c2 &x2,
                                             c2 &x3)
 {
     const c2 p = caxpy(k2, u2, a0), q = caxpy(-k2, u2, a0), e = cadd(u1, u3), f = csub(u1, u3);
     x0 = caxpy(k1, e, p);
     x2 = caxpy(-k1, e, p);
-    x1 = caxpy_i<SIGN>(k1, f, q);
-    x3 = caxpy_i<-SIGN>(k1, f, q);
+    x1 = caxpy_i<+1>(k1, f, q);
+    x3 = caxpy_i<-1>(k1, f, q);
 }
 
-template <int SIGN>
 __device__ __forceinline__ void dft2(c2 *v)
 {
     const c2 a = v[0], b = v[1];
@@ -131,49 +128,34 @@ constexpr float kR2 = 0.70710678118654752440f;  // 1 / sqrt 2
 constexpr float kC1 = 0.92387953251128675613f;  // cos(pi / 8)
 constexpr float kT1 = 0.41421356237309504880f;  // tan(pi / 8)
 
-// (1 + SIGN i) a
-template <int SIGN>
-__device__ __forceinline__ c2 one_i(c2 a) { return cadd_i<SIGN>(a, a); }
-// (-1 + SIGN i) a
-template <int SIGN>
-__device__ __forceinline__ c2 mone_i(c2 a)
-{
-    if constexpr (SIGN > 0)  // (-re - im, re - im)
-        return {sub2(mul2(dup(-1.f), a.re), a.im), sub2(a.re, a.im)};
-    else  // (im - re, -re - im)
-        return {sub2(a.im, a.re), sub2(mul2(dup(-1.f), a.re), a.im)};
-}
-// (1 + SIGN i t) a and (t + SIGN i) a
-template <int SIGN>
-__device__ __forceinline__ c2 one_it(float t, c2 a) { return caxpy_i<SIGN>(t, a, a); }
-template <int SIGN>
+// (1 + i) a
+__device__ __forceinline__ c2 one_i(c2 a) { return cadd_i<+1>(a, a); }
+// (-1 + i) a
+__device__ __forceinline__ c2 mone_i(c2 a) { return {sub2(mul2(dup(-1.f), a.re), a.im), sub2(a.re, a.im)}; }
+// (1 + i t) a and (t + i) a
+__device__ __forceinline__ c2 one_it(float t, c2 a) { return caxpy_i<+1>(t, a, a); }
 __device__ __forceinline__ c2 t_i(float t, c2 a)
 {
     const f2 k = dup(t);
-    if constexpr (SIGN > 0)
-        return {sub2(mul2(k, a.re), a.im), fma2(k, a.im, a.re)};
-    else
-        return {fma2(k, a.re, a.im), sub2(mul2(k, a.im), a.re)};
+    return {sub2(mul2(k, a.re), a.im), fma2(k, a.im, a.re)};
 }
 
-template <int SIGN>
-__device__ __forceinline__ void dft4v(c2 *v) { dft4<SIGN>(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ void dft4v(c2 *v) { dft4(v[0], v[1], v[2], v[3]); }
 
-template <int SIGN>
 __device__ __forceinline__ void dft8(c2 *v)
 {
     c2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
     c2 o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
-    dft4<SIGN>(e0, e1, e2, e3);
-    dft4<SIGN>(o0, o1, o2, o3);
-    // W8^1 = (1 + SIGN i)/sqrt2, W8^2 = SIGN i, W8^3 = (-1 + SIGN i)/sqrt2
-    const c2 u1 = one_i<SIGN>(o1), u3 = mone_i<SIGN>(o3);
+    dft4(e0, e1, e2, e3);
+    dft4(o0, o1, o2, o3);
+    // W8^1 = (1 + i)/sqrt2, W8^2 = i, W8^3 = (-1 + i)/sqrt2
+    const c2 u1 = one_i(o1), u3 = mone_i(o3);
     v[0] = cadd(e0, o0);
     v[4] = csub(e0, o0);
     v[1] = caxpy(kR2, u1, e1);
     v[5] = caxpy(-kR2, u1, e1);
-    v[2] = cadd_i<SIGN>(e2, o2);
-    v[6] = cadd_i<-SIGN>(e2, o2);
+    v[2] = cadd_i<+1>(e2, o2);
+    v[6] = cadd_i<-1>(e2, o2);
     v[3] = caxpy(kR2, u3, e3);
     v[7] = caxpy(-kR2, u3, e3);
 }
@@ -181,55 +163,54 @@ __device__ __forceinline__ void dft8(c2 *v)
 // 16 points: four radix-4 butterflies, twiddles W16^(qs) with their common
 // factor (cos pi/8 or 1/sqrt 2) left to the FMAs of the second radix-4 level:
 // 142 packed operations instead of 160
-template <int SIGN>
 __device__ __forceinline__ void dft16(c2 *v)
 {
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-        dft4<SIGN>(v[q], v[q + 4], v[q + 8], v[q + 12]);
+        dft4(v[q], v[q + 4], v[q + 8], v[q + 12]);
     c2 o[16];
     o[0] = v[0];
     o[4] = v[1];
     o[8] = v[2];
     o[12] = v[3];
-    dft4<SIGN>(o[0], o[4], o[8], o[12]);
+    dft4(o[0], o[4], o[8], o[12]);
     // s = 1: W^1 = C(1 + iT), W^2 = R(1 + i), W^3 = C(T + i)
-    dft4_scaled<SIGN>(v[4], one_it<SIGN>(kT1, v[5]), one_i<SIGN>(v[6]), t_i<SIGN>(kT1, v[7]), kC1, kR2, o[1], o[5],
+    dft4_scaled(v[4], one_it(kT1, v[5]), one_i(v[6]), t_i(kT1, v[7]), kC1, kR2, o[1], o[5],
                       o[9], o[13]);
     // s = 2: W^2, W^4 = i, W^6 = R(-1 + i)
     {
-        const c2 u1 = one_i<SIGN>(v[9]), u3 = mone_i<SIGN>(v[11]);
-        const c2 p = cadd_i<SIGN>(v[8], v[10]), q = cadd_i<-SIGN>(v[8], v[10]), e = cadd(u1, u3), f = csub(u1, u3);
+        const c2 u1 = one_i(v[9]), u3 = mone_i(v[11]);
+        const c2 p = cadd_i<+1>(v[8], v[10]), q = cadd_i<-1>(v[8], v[10]), e = cadd(u1, u3), f = csub(u1, u3);
         o[2] = caxpy(kR2, e, p);
         o[10] = caxpy(-kR2, e, p);
-        o[6] = caxpy_i<SIGN>(kR2, f, q);
-        o[14] = caxpy_i<-SIGN>(kR2, f, q);
+        o[6] = caxpy_i<+1>(kR2, f, q);
+        o[14] = caxpy_i<-1>(kR2, f, q);
     }
     // s = 3: W^3 = C(T + i), W^6 = R(-1 + i), W^9 = -C(1 + iT)
     {
-        const c2 u1 = t_i<SIGN>(kT1, v[13]), u2 = mone_i<SIGN>(v[14]), u3 = one_it<SIGN>(kT1, v[15]);
+        const c2 u1 = t_i(kT1, v[13]), u2 = mone_i(v[14]), u3 = one_it(kT1, v[15]);
         const c2 p = caxpy(kR2, u2, v[12]), q = caxpy(-kR2, u2, v[12]), e = csub(u1, u3), f = cadd(u1, u3);
         o[3] = caxpy(kC1, e, p);
         o[11] = caxpy(-kC1, e, p);
-        o[7] = caxpy_i<SIGN>(kC1, f, q);
-        o[15] = caxpy_i<-SIGN>(kC1, f, q);
+        o[7] = caxpy_i<+1>(kC1, f, q);
+        o[15] = caxpy_i<-1>(kC1, f, q);
     }
 #pragma unroll
     for (int i = 0; i < 16; ++i)
         v[i] = o[i];
 }
 
-template <int R, int SIGN>
+template <int R>
 __device__ __forceinline__ void dft(c2 *v)
 {
     if constexpr (R == 2)
-        dft2<SIGN>(v);
+        dft2(v);
     else if constexpr (R == 4)
-        dft4v<SIGN>(v);
+        dft4v(v);
     else if constexpr (R == 8)
-        dft8<SIGN>(v);
+        dft8(v);
     else
-        dft16<SIGN>(v);
+        dft16(v);
 }
 
 __device__ __forceinline__ float4 to4(c2 v)
@@ -316,7 +297,7 @@ __device__ __forceinline__ void stage_store(const c2 (&v)[16], float4 *__restric
 }
 
 // This thread's twiddles of stage S (PairFft::words), from a table tw[e] =
-// exp(2 pi i SIGN e / NTAB) (NTAB a multiple of N); further words are zero.
+// exp(2 pi i e / NTAB) (NTAB a multiple of N); further words are zero.
 template <int LOG2N, int S, int NTAB>
 __device__ __forceinline__ void stage_twiddles(float (&w)[32], int tid, const float2 *__restrict__ tw)
 {
@@ -358,7 +339,7 @@ __device__ __forceinline__ void twiddle_out(c2 (&v)[16], const float (&w)[32])
 
 // The last stage: input twiddles, butterflies.  Register slot q R + r then
 // holds output m = tid + q T + r N/R (last_out_index).
-template <int LOG2N, int SIGN>
+template <int LOG2N>
 __device__ __forceinline__ void last_stage(c2 (&v)[16], const float (&w)[32])
 {
     using F = FftShape<LOG2N>;
@@ -370,7 +351,7 @@ __device__ __forceinline__ void last_stage(c2 (&v)[16], const float (&w)[32])
             const int i = q * (R - 1) + r - 1;
             v[q * R + r] = ctw(v[q * R + r], w[2 * i], w[2 * i + 1]);
         }
-        dft<R, SIGN>(&v[q * R]);
+        dft<R>(&v[q * R]);
     }
 }
 

@@ -131,13 +131,13 @@ __device__ __forceinline__ void pair_ifft(c2 (&v)[16], float4 *buf, int g, int j
     if constexpr (P::X::words(S) > 0)
         load_twiddles<LOG2N, S>(w, tm);
     if constexpr (S + 1 < NST) {
-        pairfft::dft16<+1>(v);
+        pairfft::dft16(v);
         if constexpr (P::X::words(S) > 0)
             twiddle_out(v, w);
         stage_store<P::LT, S>(v, buf, j);
         pair_ifft<LOG2N, S + 1>(v, buf, g, j, tm);
     } else {
-        last_stage<P::LT, +1>(v, w);
+        last_stage<P::LT>(v, w);
     }
 }
 

@@ -421,12 +421,11 @@ __device__ __forceinline__ void issue_gemm2(uint32_t tmem, uint32_t s0, uint32_t
 // Thread 0 waits for a commit (bounded); every thread learns the outcome.
 // Returns false (uniformly) on a timeout; parity then still names the
 // phase waited for.
-__device__ __forceinline__ bool wait_gemm(int tid, uint32_t bar, uint32_t &parity,
-                                          unsigned long long limit_ns = kWaitLimitNs)
+__device__ __forceinline__ bool wait_gemm(int tid, uint32_t bar, uint32_t &parity)
 {
     bool ok = true;
     if (tid == 0)
-        ok = mbar_wait(bar, parity, limit_ns);
+        ok = mbar_wait(bar, parity, kWaitLimitNs);
     const bool failed = __syncthreads_or(!ok);
     if (!failed)
         parity ^= 1;
@@ -447,7 +446,7 @@ __device__ __forceinline__ void pow2_scale_to(float mx, float &s, float &inv)
 // A bin pair of the spectrum ring.  Nothing of the ring is read twice by an
 // SM before it has left L1, so at 8192 and 16384 points it goes past L1, which
 // then keeps the tables that are (the filter, read with every step at 16384):
-// 1.4 and 4 % off.  At 4096 the same costs 1.5 %.
+// 1.5 and 3.6 % off.  At 4096 the same costs 1.5 %.
 template <int LOG2N>
 __device__ __forceinline__ float4 ring_load(const float4 *p)
 {
