@@ -417,6 +417,10 @@ MSOSM_API msosm_status msosm_writer_close(msosm_writer *w, unsigned long long *b
  * generate_pulsar_signal(pinned = true) allocates) or plain malloc. */
 MSOSM_API msosm_status msosm_host_alloc(size_t bytes, int pinned, void **out);
 MSOSM_API msosm_status msosm_host_free(void *p, int pinned);
+/* The calling thread's CUDA context (the current device's, made where there is
+ * none yet) as a number never given twice in a process: page-locked memory ends
+ * with its context when a program resets the device. */
+MSOSM_API msosm_status msosm_context_id(unsigned long long *id);
 
 /* Random numbers of every simulator: Philox4x32-10 (Salmon et al., SC11,
  * 2011) at counter (lo(i), hi(i), tag, 0) under the key (lo(seed), hi(seed))

@@ -174,6 +174,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "msosm_cnn_gradient": (i32, [vp, vp, vp, vp, i32, ctypes.POINTER(f32), vp]),
         "msosm_cnn_adam_step": (i32, [vp, f32]),
         "msosm_host_alloc": (i32, [ctypes.c_size_t, i32, pvp]),
+        "msosm_context_id": (i32, [ctypes.POINTER(ctypes.c_ulonglong)]),
         "msosm_host_free": (i32, [vp, i32]),
         "msosm_sim_normals": (i32, [ull, ull, ul, u32, vp, vp]),
         "msosm_sim_awgn": (i32, [ull, ul, i32, f32, f32, f32, vp]),

@@ -10,8 +10,8 @@ rewritten by a later result while the caller's own asynchronous copy out of it
 was still under way, and a forked process would share it with its parent.
 
 ``empty`` hands out arrays over page-locked blocks; when an array and every view
-of it are gone its block goes back to a pool (at most POOL_BYTES in all, handed
-out or waiting; beyond that, and for small or large sizes, the array is an
+of it are gone its block goes back to a pool (at most POOL_BYTES per CUDA context,
+handed out or waiting; beyond that, and for small or large sizes, the array is an
 ordinary one).  Safe to use from several threads.
 """
 from __future__ import annotations
@@ -29,6 +29,8 @@ POOL_BYTES = 16 << 20
 _lock = threading.RLock()  # re-entrant: an array may be collected while the pool is in use
 _free: "dict[int, list]" = {}  # block size -> addresses
 _total = 0                     # bytes of all blocks
+_context = 0                   # the CUDA context (msosm_context_id) these belong to
+_others: "dict[int, tuple]" = {}  # _free and _total of other contexts
 
 
 def _take(size: int):
@@ -52,18 +54,33 @@ def _take(size: int):
         return p.value
 
 
+def _follow_context() -> None:
+    """Switch to the current context's blocks.  Those of a context that is gone
+    (a program that resets the device takes its page-locked memory with it) are
+    never handed out again: ids do not come back.  Under the lock."""
+    global _context, _free, _total
+    from ._abi import check, lib
+    now = ctypes.c_ulonglong()
+    check(lib().msosm_context_id(ctypes.byref(now)))
+    if now.value != _context:
+        _others[_context] = (_free, _total)
+        _context = now.value
+        _free, _total = _others.pop(_context, ({}, 0))
+
+
 class _Block:
     """Owner of a block for as long as an array refers to it."""
 
     def __init__(self, address: int, size: int, shape, dtype):
-        self._address, self._size = address, size
+        self._address, self._size, self._context = address, size, _context
         self.__array_interface__ = {"data": (address, False), "shape": tuple(shape), "typestr": np.dtype(dtype).str,
                                     "version": 3}
 
     def __del__(self):
         try:
             with _lock:
-                _free.setdefault(self._size, []).append(self._address)
+                mine = _free if self._context == _context else _others[self._context][0]
+                mine.setdefault(self._size, []).append(self._address)
         except Exception:  # interpreter shutdown
             pass
 
@@ -83,6 +100,8 @@ def empty(shape, dtype) -> np.ndarray:
 def fetch(shape, dtype, read) -> np.ndarray:
     """A new array of ordinary memory that read(address) has filled; read
     returns when its copy is done."""
-    a = empty(shape, dtype)
+    with _lock:
+        _follow_context()
+        a = empty(shape, dtype)
     read(a.ctypes.data)
     return a.copy() if isinstance(a.base, _Block) else a

@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <new>
 #include <string>
 #include <memory>
@@ -79,7 +80,7 @@ bool is_device_ptr(const void *p)
 template <typename T>
 T *mapped_host(T *p, size_t n)
 {
-    if (!host_blocks().covers(p, n * sizeof(T)))
+    if (!host_blocks().covers(p, n * sizeof(T), context_id()))
         return nullptr;
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
@@ -161,6 +162,7 @@ struct msosm_dedisp {
     bool tc = false, tc_bf16 = false;
     int *status_d = nullptr;
     int *status_h = nullptr;  // page-locked: the status as of the last synchronising call
+    unsigned long long status_ctx = 0;  // the context it belongs to
     long long tc_wait_limit_ns = kTcWaitLimitDefaultNs;  // each wait of the kernel on a GEMM
     float *row_max = nullptr;  // [S] largest |component| of each ring row
     float *h_max = nullptr;    // [D] largest |component| of each trial's H
@@ -186,30 +188,44 @@ namespace {
 
 // Page-locked words for the handles' status: slots of 4 KB pages (a page-locked
 // allocation costs about a millisecond), taken and given back under a lock; a
-// page per 1024 handles alive at one time.
+// page per 1024 handles alive at one time in a context, whose end is theirs too.
+struct StatusSlots {
+    std::vector<int *> free;
+    size_t all = 0;  // slots of the context's pages
+};
 std::mutex g_slot_lock;
-std::vector<int *> g_slots;
+std::map<unsigned long long, StatusSlots> g_slots;  // by context_id()
 
-cudaError_t status_slot(int **out)
+cudaError_t status_slot(int **out, unsigned long long *ctx)
 {
+    *ctx = context_id();
     const std::lock_guard<std::mutex> lock(g_slot_lock);
-    if (g_slots.empty()) {
-        int *page = nullptr;
-        const cudaError_t e = cudaHostAlloc((void **)&page, 1024 * sizeof(int), cudaHostAllocPortable);
-        if (e != cudaSuccess)
-            return e;
-        for (int i = 1023; i >= 0; --i)
-            g_slots.push_back(page + i);
+    try {
+        StatusSlots &s = g_slots[*ctx];
+        if (s.free.empty()) {
+            s.free.reserve(s.all + 1024);  // giving back never allocates
+            int *page = nullptr;
+            const cudaError_t e = cudaHostAlloc((void **)&page, 1024 * sizeof(int), cudaHostAllocPortable);
+            if (e != cudaSuccess)
+                return e;
+            s.all += 1024;
+            for (int i = 1023; i >= 0; --i)
+                s.free.push_back(page + i);
+        }
+        *out = s.free.back();
+        s.free.pop_back();
+        return cudaSuccess;
+    } catch (const std::bad_alloc &) {
+        return cudaErrorMemoryAllocation;
     }
-    *out = g_slots.back();
-    g_slots.pop_back();
-    return cudaSuccess;
 }
 
-void status_slot_free(int *slot)
+void status_slot_free(int *slot, unsigned long long ctx)
 {
     const std::lock_guard<std::mutex> lock(g_slot_lock);
-    g_slots.push_back(slot);
+    const auto it = g_slots.find(ctx);
+    if (it != g_slots.end())
+        it->second.free.push_back(slot);
 }
 
 void release(msosm_dedisp *d)
@@ -231,7 +247,7 @@ void release(msosm_dedisp *d)
     if (d->span_host)
         cudaFreeHost(d->span_host);
     if (d->status_h)
-        status_slot_free(d->status_h);
+        status_slot_free(d->status_h, d->status_ctx);
     for (int i = 0; i < 2; ++i) {
         if (d->ev_copied[i])
             cudaEventDestroy(d->ev_copied[i]);
@@ -867,7 +883,7 @@ msosm_status msosm_dedisp_create(const float *bw, const float *dm, const float *
             CKD(e);
             CKD(dalloc(&d->status_d, 1, tot));
             CKD(cudaMemset(d->status_d, 0, sizeof(int)));
-            CKD(status_slot(&d->status_h));
+            CKD(status_slot(&d->status_h, &d->status_ctx));
             // scale bounds: ring rows not yet written hold zero
             CKD(dalloc(&d->row_max, (size_t)d->S, tot));
             CKD(cudaMemset(d->row_max, 0, sizeof(float) * d->S));

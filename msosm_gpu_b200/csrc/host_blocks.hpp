@@ -13,19 +13,19 @@ namespace msosm {
 
 class HostBlocks {
 public:
-    // may throw std::bad_alloc
-    void add(const void *p, size_t bytes)
+    // a block of the context ctx (context_id()); may throw std::bad_alloc
+    void add(const void *p, size_t bytes, unsigned long long ctx)
     {
         const std::lock_guard<std::mutex> lock(m_);
-        blocks_[(uintptr_t)p] = bytes;
+        blocks_[(uintptr_t)p] = {bytes, ctx};
     }
     void remove(const void *p)
     {
         const std::lock_guard<std::mutex> lock(m_);
         blocks_.erase((uintptr_t)p);
     }
-    // whether [p, p + bytes) lies in one block
-    bool covers(const void *p, size_t bytes) const
+    // whether [p, p + bytes) lies in one block of the context ctx
+    bool covers(const void *p, size_t bytes, unsigned long long ctx) const
     {
         const std::lock_guard<std::mutex> lock(m_);
         auto it = blocks_.upper_bound((uintptr_t)p);
@@ -33,12 +33,16 @@ public:
             return false;
         --it;
         const uintptr_t at = (uintptr_t)p - it->first;
-        return at <= it->second && bytes <= it->second - at;
+        return it->second.ctx == ctx && at <= it->second.bytes && bytes <= it->second.bytes - at;
     }
 
 private:
+    struct Block {
+        size_t bytes;
+        unsigned long long ctx;
+    };
     mutable std::mutex m_;
-    std::map<uintptr_t, size_t> blocks_;
+    std::map<uintptr_t, Block> blocks_;
 };
 
 HostBlocks &host_blocks();  // sim.cu

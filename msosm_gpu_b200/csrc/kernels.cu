@@ -27,6 +27,7 @@
 #include <mutex>
 #include <utility>
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 namespace msosm {
@@ -513,24 +514,36 @@ size_t fft_smem_bytes()
     return (use_pingpong<LOG2N>() ? 2 : 1) * F::SMEM * sizeof(float2);
 }
 
+unsigned long long context_id()
+{
+    using GetId = CUresult (*)(CUcontext, unsigned long long *);
+    static const GetId get = [] {
+        void *f = nullptr;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault) != cudaSuccess)
+            cudaGetLastError();
+        return reinterpret_cast<GetId>(f);
+    }();
+    unsigned long long id = 0;
+    return get && get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
 cudaError_t allow_smem(const void *kernel, size_t bytes, bool max_carveout)
 {
     static std::mutex m;
-    static std::map<std::pair<const void *, int>, size_t> allowed;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess)
-        return e;
+    static std::map<std::pair<const void *, unsigned long long>, size_t> allowed;
+    const unsigned long long ctx = context_id();
     const std::lock_guard<std::mutex> lock(m);
-    const auto it = allowed.find({kernel, dev});
-    if (it != allowed.end() && it->second >= bytes)
-        return cudaSuccess;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (ctx) {
+        const auto it = allowed.find({kernel, ctx});
+        if (it != allowed.end() && it->second >= bytes)
+            return cudaSuccess;
+    }
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e == cudaSuccess && max_carveout)
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  (int)cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess)
-        allowed[{kernel, dev}] = bytes;
+    if (e == cudaSuccess && ctx)
+        allowed[{kernel, ctx}] = bytes;
     return e;
 }
 

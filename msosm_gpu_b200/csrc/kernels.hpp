@@ -115,9 +115,14 @@ struct DesignArgs {
 
 bool log2n_supported(int log2n);
 
+// The current context's id, never given twice in a process; 0 without one.
+// What the process keeps for a context (attributes, page-locked memory) ends with
+// it when the program resets the device, so it is kept by this id.
+unsigned long long context_id();
+
 // Allows a kernel `bytes` of dynamic shared memory on the current device (and,
 // max_carveout, asks for the largest shared-memory carveout).  The attribute is
-// raised once per kernel and device and kept; any thread may ask.
+// raised once per kernel and context and kept; any thread may ask.
 cudaError_t allow_smem(const void *kernel, size_t bytes, bool max_carveout = false);
 template <typename... A>
 cudaError_t allow_smem(void (*kernel)(A...), size_t bytes, bool max_carveout = false)

@@ -379,7 +379,7 @@ msosm_status msosm_host_alloc(size_t bytes, int pinned, void **out)
             return sim_cuda_fail(e, "cudaMallocHost");
         }
         try {
-            host_blocks().add(*out, bytes ? bytes : 1);
+            host_blocks().add(*out, bytes ? bytes : 1, context_id());
         } catch (const std::bad_alloc &) {
             cudaFreeHost(*out);
             *out = nullptr;
@@ -389,6 +389,20 @@ msosm_status msosm_host_alloc(size_t bytes, int pinned, void **out)
     }
     *out = std::malloc(bytes ? bytes : 1);
     return *out ? MSOSM_OK : sim_fail(MSOSM_ERR_OOM, "host allocation");
+}
+
+msosm_status msosm_context_id(unsigned long long *id)
+{
+    if (!id)
+        return sim_fail(MSOSM_ERR_BAD_ARG, "null argument");
+    *id = context_id();
+    if (*id == 0) {  // a thread that has called nothing yet
+        const cudaError_t e = cudaFree(nullptr);
+        if (e != cudaSuccess)
+            return sim_cuda_fail(e, "context");
+        *id = context_id();
+    }
+    return MSOSM_OK;
 }
 
 msosm_status msosm_host_free(void *p, int pinned)

@@ -24,6 +24,12 @@ class FakeLib:
         del self.blocks[p.value]
         return 0
 
+    context = 7
+
+    def msosm_context_id(self, out):
+        out._obj.value = self.context
+        return 0
+
 
 @pytest.fixture
 def fake(monkeypatch):
@@ -31,6 +37,8 @@ def fake(monkeypatch):
     monkeypatch.setattr(_abi, "lib", lambda: f)
     monkeypatch.setattr(_pinned, "_free", {})
     monkeypatch.setattr(_pinned, "_total", 0)
+    monkeypatch.setattr(_pinned, "_context", f.context)
+    monkeypatch.setattr(_pinned, "_others", {})
     yield f
     gc.collect()
 
